@@ -7,14 +7,15 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_native")
 LIB = os.path.join(OUT_DIR, "libklon3d_b200.so")
-SOURCES = ["k3d_step.cu", "k3d_step_f32.cu", "k3d_build.cu", "k3d_host.cpp", "scene_build.cpp", "k3d_noalloc.cu", "k3d_selbst.cu",
+SOURCES = ["k3d_step.cu", "k3d_kachel.cu", "k3d_plan.cpp", "k3d_step_f32.cu", "k3d_build.cu", "k3d_host.cpp", "scene_build.cpp", "k3d_noalloc.cu", "k3d_selbst.cu",
            "k3d_selbst_host.cpp", "k3d_adjoint.cu", "k3d_netz.cu"]
-HEADERS = ["k3d_step.h", "k3d_device.cuh", "k3d_step_common.cuh", "k3d_solve.cuh", "scene_build.h", "k3d_selbst.h",
+HEADERS = ["k3d_step.h", "k3d_device.cuh", "k3d_step_common.cuh", "k3d_solve.cuh", "k3d_plan.h", "scene_build.h", "k3d_selbst.h",
            "k3d_selbst_host.h", "k3d_adjoint.h", "k3d_vec.cuh", "k3d_netz.cuh", "k3d_netz.h"]
 # Per-file flags. The build of the system and the self-collision stage round
 # every product and sum on their own (no fused multiply-add), as the
@@ -26,7 +27,7 @@ HEADERS = ["k3d_step.h", "k3d_device.cuh", "k3d_step_common.cuh", "k3d_solve.cuh
 # adjoint replays the forward's contact queries and rounds the same way; the
 # body mesh's nearest-point regions and distances round as the reference's;
 # the allocation-free operator evaluates the same element products as the build.
-EXTRA = {"k3d_step.cu": ["-fmad=false"], "k3d_build.cu": ["-fmad=false"], "k3d_selbst.cu": ["-fmad=false"], "k3d_adjoint.cu": ["-fmad=false"],
+EXTRA = {"k3d_step.cu": ["-fmad=false"], "k3d_kachel.cu": ["-fmad=false"], "k3d_build.cu": ["-fmad=false"], "k3d_selbst.cu": ["-fmad=false"], "k3d_adjoint.cu": ["-fmad=false"],
          "k3d_netz.cu": ["-fmad=false"], "k3d_noalloc.cu": ["-fmad=false"]}
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -52,8 +53,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     obj_dir = os.path.join(OUT_DIR, "obj")
     os.makedirs(obj_dir, exist_ok=True)
-    objs = []
-    for f in SOURCES:
+
+    def compile_one(f):
         p = os.path.join(CSRC, f)
         o = os.path.join(obj_dir, f + ".o")
         lang = ["-x", "cu"] if f.endswith(".cpp") else []
@@ -62,7 +63,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))
         subprocess.run(cmd, check=True, cwd=CSRC)
-        objs.append(o)
+        return o
+
+    with ThreadPoolExecutor(max_workers=min(len(SOURCES), os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(compile_one, SOURCES))
     link = [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-cudart", "shared",
             "-o", LIB + ".tmp", *objs]
     subprocess.run(link, check=True, cwd=CSRC)

@@ -294,7 +294,33 @@ __global__ void __launch_bounds__(kBlock) adj_final_set_kernel(const __grid_cons
   }
 }
 
-// y = A x on the assembled FP64 blocks
+// y = A x on the assembled FP64 blocks (slabs: a thread per position)
+__global__ void __launch_bounds__(kBlock) adj_spmv_kachel_kernel(const __grid_constant__ StepArgs a, const double* x,
+                                                                  double* y) {
+  K3D_FOR(p, 32 * a.ka_slices) {
+    const uint32_t z = __ldg(&a.ka_row[p]);
+    if (z == 0xffffffffu) continue;
+    const uint4 sl = __ldg(&a.ka_slice[p >> 5]);
+    const int l = int(p & 31);
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    for (uint32_t k = 0; k < sl.y + sl.w; ++k) {
+      const size_t slab = k < sl.y ? sl.x + k : sl.z + (k - sl.y);
+      const uint32_t c = __ldg(&a.col[slab * 32 + l]);
+      if (c == 0xffffffffu) break;
+      const char* satz = static_cast<const char*>(a.bmat) + slab * kachel_satz(sizeof(double));
+      const D3 q = ld3(x, c & 0x7fffffffu);
+      const R4<double> u = reinterpret_cast<const R4<double>*>(satz)[l];
+      const R4<double> v = reinterpret_cast<const R4<double>*>(satz + 128 * sizeof(double))[l];
+      const double w = reinterpret_cast<const double*>(satz + 256 * sizeof(double))[l];
+      sx += u.x * q.x + u.y * q.y + u.z * q.z;
+      sy += u.w * q.x + v.x * q.y + v.y * q.z;
+      sz += v.z * q.x + v.w * q.y + w * q.z;
+    }
+    st3(y, z & 0x7fffffffu, d3(sx, sy, sz));
+  }
+}
+
+// y = A x on the assembled FP64 blocks (ELL rows)
 __global__ void __launch_bounds__(kBlock) adj_spmv_kernel(const __grid_constant__ StepArgs a, const double* x,
                                                            double* y) {
   const R4<double>* b4 = static_cast<const R4<double>*>(a.bmat);
@@ -592,6 +618,7 @@ cudaError_t launch_adjoint_step(const StepArgs& a0, const AdjArgs& j, int blocks
   auto spmv = [&](const double* x, double* y) {
     void* as[] = {(void*)&a, (void*)&x, (void*)&y};
     ++launched;
+    if (a.ka_blk) return grid((const void*)adj_spmv_kachel_kernel, as, 32 * a.ka_slices, st);
     return grid((const void*)adj_spmv_kernel, as, a.n, st);
   };
   // the system at the recorded input state, with the final contact set

@@ -338,9 +338,23 @@ __global__ void __launch_bounds__(kBlock) assemble_kernel(const __grid_constant_
   const double* sk = static_cast<const double*>(own ? a.s_k : a.s_k64);
   R* bm = static_cast<R*>(a.bmat);
   const double h2 = a.h * a.h;
+  const bool kachel = a.ka_blk != nullptr;
   K3D_FOR(sid, a.bplane) {
-    const int64_t i = sid % a.np, k = sid / a.np;
-    if (i >= a.n || k >= int64_t(__ldg(&a.row_cnt[i]))) continue;
+    int64_t i;  // the row, on a diagonal block (elsewhere not needed)
+    bool diag;
+    if (kachel) {  // slab sid / 32, lane sid % 32
+      const uint32_t c = __ldg(&a.col[sid]);
+      char* satz = static_cast<char*>(a.bmat) + size_t(sid >> 5) * kachel_satz(sizeof(R));
+      reinterpret_cast<uint16_t*>(satz + 288 * sizeof(R))[sid & 31] = __ldg(&a.ka_lc[sid]);
+      if (c == 0xffffffffu) continue;
+      i = int64_t(c & 0x7fffffffu);
+      diag = (c >> 31) != 0;
+    } else {
+      i = sid % a.np;
+      const int64_t k = sid / a.np;
+      if (i >= a.n || k >= int64_t(__ldg(&a.row_cnt[i]))) continue;
+      diag = int64_t(__ldg(&a.col[sid])) == i;
+    }
     double B[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (uint32_t e = __ldg(&a.ctr_off[sid]); e < __ldg(&a.ctr_off[sid + 1]); ++e) {
       const uint32_t code = __ldg(&a.ctr[e]);
@@ -393,13 +407,21 @@ __global__ void __launch_bounds__(kBlock) assemble_kernel(const __grid_constant_
           for (int c = 0; c < 3; ++c) B[3 * r + c] += kk * (nv[r] * nv[c] * (1.0 - dq.w) + (r == c ? dq.w : 0.0));
       }
     }
-    if (int64_t(__ldg(&a.col[sid])) == i) {
+    if (diag) {
       const double md = a.masse[i] * (1.0 + a.h * a.daempf);
       B[0] += md;
       B[4] += md;
       B[8] += md;
     }
     // the block as two 4-vectors (m00 m01 m02 m10), (m11 m12 m20 m21) and m22
+    if (kachel) {
+      char* satz = reinterpret_cast<char*>(bm) + size_t(sid >> 5) * kachel_satz(sizeof(R));
+      const int l = int(sid & 31);
+      reinterpret_cast<R4<R>*>(satz)[l] = R4<R>{R(B[0]), R(B[1]), R(B[2]), R(B[3])};
+      reinterpret_cast<R4<R>*>(satz + 128 * sizeof(R))[l] = R4<R>{R(B[4]), R(B[5]), R(B[6]), R(B[7])};
+      reinterpret_cast<R*>(satz + 256 * sizeof(R))[l] = R(B[8]);
+      continue;
+    }
     R4<R>* b4 = reinterpret_cast<R4<R>*>(bm);
     b4[sid] = R4<R>{R(B[0]), R(B[1]), R(B[2]), R(B[3])};
     b4[a.bplane + sid] = R4<R>{R(B[4]), R(B[5]), R(B[6]), R(B[7])};

@@ -13,6 +13,7 @@
 #include "../../include/klon3d_step.h"
 #include "k3d_adjoint.h"
 #include "k3d_netz.h"
+#include "k3d_plan.h"
 #include "k3d_selbst_host.h"
 #include "k3d_step.h"
 #include "scene_build.h"
@@ -45,6 +46,7 @@ struct k3d_solver {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err, name;
   int blocks = 0;
+  size_t ka_smem = 0;  // shared memory a CTA of the tiled PCG takes (0: the launch over ELL rows)
   size_t rsize = 8;  // operator records, assembled blocks, preconditioner
   size_t vsize = 8;  // the PCG's vectors
   uint8_t* d_fest = nullptr;  // device copy of a caller's contact set
@@ -101,69 +103,34 @@ static k3d_status cuda_fail(k3d_solver* h, cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail((h), e_, #call); \
   } while (0)
 
-// Block pattern of A (3x3 blocks): per point its sorted columns, ELL layout
-// with block (rank k, row i) at k * np + i; per block the element
-// contributions in a fixed order (membranes, then bends, then springs, each in
-// element order, then by corner pair). Code: type << 30 | a << 28 | b << 26 | id.
+// The blocks of A as the device stores them: slabs of the tiled PCG, or ELL
+// rows (block (rank k, row i) at k * np + i).
 struct Pattern {
-  std::vector<uint32_t> cnt, col, ctr_off, ctr;
-  size_t kmax = 0;
+  std::vector<uint32_t> cnt, col, ctr_off, ctr;  // cnt: ELL rows' blocks
+  size_t kmax = 0, plane = 0;                    // plane: block slots (32 per slab)
+  bool kachel = false;
+  Kachelplan plan;
 };
 
-static bool build_pattern(size_t n, size_t np, const uint32_t* m_p, size_t nt, const uint32_t* b_p, size_t nb,
-                          const std::vector<uint4>& s_idx, Pattern& P) {
-  if (nt >= (size_t(1) << 26) || nb >= (size_t(1) << 26) || s_idx.size() >= (size_t(1) << 26)) return false;
-  std::vector<std::vector<uint32_t>> cols(n);
-  for (size_t i = 0; i < n; ++i) cols[i].push_back(uint32_t(i));
-  auto link = [&](const uint32_t* q, int k) {
-    for (int a = 0; a < k; ++a)
-      for (int b = 0; b < k; ++b) cols[q[a]].push_back(q[b]);
-  };
-  for (size_t t = 0; t < nt; ++t) link(m_p + 3 * t, 3);
-  for (size_t b = 0; b < nb; ++b) link(b_p + 4 * b, 4);
-  for (const uint4& q : s_idx) {
-    const uint32_t ij[2] = {q.x, q.y};
-    link(ij, 2);
+static bool build_pattern(const Elemente& E, const Spalten& S, size_t np, Pattern& P) {
+  if (E.nt >= (size_t(1) << 26) || E.nb >= (size_t(1) << 26) || E.ns >= (size_t(1) << 26)) return false;
+  if (P.kachel) {
+    P.plane = P.plan.slabs * 32;
+    beitraege(E, S, P.plane, [&](size_t i, uint32_t k) { return P.plan.slot(i, k); }, P.ctr_off, P.ctr);
+    return true;
   }
-  P.cnt.assign(n, 0);
+  P.cnt.resize(E.n);
   P.kmax = 0;
-  for (size_t i = 0; i < n; ++i) {
-    std::sort(cols[i].begin(), cols[i].end());
-    cols[i].erase(std::unique(cols[i].begin(), cols[i].end()), cols[i].end());
-    P.cnt[i] = uint32_t(cols[i].size());
-    P.kmax = std::max(P.kmax, cols[i].size());
+  for (size_t i = 0; i < E.n; ++i) {
+    P.cnt[i] = S.breit(i);
+    P.kmax = std::max(P.kmax, size_t(P.cnt[i]));
   }
   if (P.kmax * np >= (size_t(1) << 32)) return false;
-  const size_t ns = P.kmax * np;
-  P.col.assign(ns, 0);
-  for (size_t i = 0; i < n; ++i)
-    for (size_t k = 0; k < cols[i].size(); ++k) P.col[k * np + i] = cols[i][k];
-  auto slot = [&](uint32_t i, uint32_t j) -> size_t {
-    const auto& c = cols[i];
-    return size_t(std::lower_bound(c.begin(), c.end(), j) - c.begin()) * np + i;
-  };
-  // count, then fill (stable: element order within a block)
-  P.ctr_off.assign(ns + 1, 0);
-  auto each = [&](auto&& f) {
-    for (size_t t = 0; t < nt; ++t)
-      for (uint32_t a = 0; a < 3; ++a)
-        for (uint32_t b = 0; b < 3; ++b)
-          f(slot(m_p[3 * t + a], m_p[3 * t + b]), (0u << 30) | (a << 28) | (b << 26) | uint32_t(t));
-    for (size_t e = 0; e < nb; ++e)
-      for (uint32_t a = 0; a < 4; ++a)
-        for (uint32_t b = 0; b < 4; ++b)
-          f(slot(b_p[4 * e + a], b_p[4 * e + b]), (1u << 30) | (a << 28) | (b << 26) | uint32_t(e));
-    for (size_t q = 0; q < s_idx.size(); ++q) {
-      const uint32_t ij[2] = {s_idx[q].x, s_idx[q].y};
-      for (uint32_t a = 0; a < 2; ++a)
-        for (uint32_t b = 0; b < 2; ++b) f(slot(ij[a], ij[b]), (2u << 30) | (a << 28) | (b << 26) | uint32_t(q));
-    }
-  };
-  each([&](size_t sl, uint32_t) { P.ctr_off[sl + 1]++; });
-  for (size_t q = 0; q < ns; ++q) P.ctr_off[q + 1] += P.ctr_off[q];
-  P.ctr.assign(P.ctr_off[ns], 0);
-  std::vector<uint32_t> fill(P.ctr_off.begin(), P.ctr_off.end() - 1);
-  each([&](size_t sl, uint32_t code) { P.ctr[fill[sl]++] = code; });
+  P.plane = P.kmax * np;
+  P.col.assign(P.plane, 0);
+  for (size_t i = 0; i < E.n; ++i)
+    for (uint32_t k = 0; k < P.cnt[i]; ++k) P.col[k * np + i] = S.sp[S.anf[i] + k];
+  beitraege(E, S, P.plane, [&](size_t i, uint32_t k) { return size_t(k) * np + i; }, P.ctr_off, P.ctr);
   return true;
 }
 
@@ -178,6 +145,10 @@ struct Carve {
   void *m_rin, *m_kgA, *m_rin64, *m_kgA64;
   double2 *b_kr, *s_kl;
   uint32_t *row_cnt, *col, *ctr_off, *ctr;
+  KachelBlk* ka_blk;
+  uint32_t *ka_row, *ka_halo;
+  uint4* ka_slice;
+  uint16_t* ka_lc;
   Grp* grp;
   uint32_t *blk_grp, *pinst;
 };
@@ -262,15 +233,34 @@ static void carve(k3d_solver* h, Arena& A, size_t N, size_t T, size_t B, size_t 
   a.pinst = cv.pinst = h->n_grp > 1 ? A.take<uint32_t>(N) : nullptr;
   a.stats = A.take<long long>(ST_COUNT);
   a.stat_rest_max = A.take<double>(2);
-  // assembled A (BSR, ELL by rank) and its contribution lists
-  const size_t nbs = P.kmax * np;
+  // assembled A (slabs or ELL rows) and its contribution lists
+  const size_t nbs = P.plane;
   a.bplane = int64_t(nbs);
-  a.row_cnt = cv.row_cnt = A.take<uint32_t>(N);
   a.col = cv.col = A.take<uint32_t>(nbs);
-  a.bmat = A.take<char>(9 * nbs * R);
   a.ctr_off = cv.ctr_off = A.take<uint32_t>(nbs + 1);
   a.ctr = cv.ctr = A.take<uint32_t>(P.ctr.size());
-  a.cw2 = A.take<char>(8 * N * V);  // the second buffer of (c, w)
+  if (P.kachel) {
+    const Kachelplan& K = P.plan;
+    a.bmat = A.take<char>(K.slabs * kachel_satz(R));
+    a.ka_blk = cv.ka_blk = A.take<KachelBlk>(K.blk.size());
+    a.ka_row = cv.ka_row = A.take<uint32_t>(K.row.size());
+    a.ka_halo = cv.ka_halo = A.take<uint32_t>(K.halo.size());
+    a.ka_slice = cv.ka_slice = A.take<uint4>(K.slice.size());
+    a.ka_lc = cv.ka_lc = A.take<uint16_t>(nbs);
+    a.ka_wort = A.take<ulonglong2>(6 * N);
+    a.ka_pv = A.take<char>(6 * 32 * K.slice.size() * R);
+    a.ka_dv = A.take<double>(3 * 32 * K.slice.size());
+    a.ka_summe = A.take<ulonglong2>(4 * size_t(kKachelKopien) * size_t(kKachelWorte));
+    a.ka_slices = int64_t(K.slice.size());
+    a.ka_blocks = K.blocks;
+    a.ka_q = K.q;
+    a.ka_smem = int(h->ka_smem);
+    a.ka_rsize = int(R);
+  } else {
+    a.row_cnt = cv.row_cnt = A.take<uint32_t>(N);
+    a.bmat = A.take<char>(9 * nbs * R);
+    a.cw2 = A.take<char>(8 * N * V);  // the second buffer of (c, w)
+  }
   cv.m_rin64 = cv.m_kgA64 = nullptr;
   if (R == 4) {  // FP64 operator records: the assembly of the FP32 blocks reads them
     a.m_f1w64 = A.take<double4>(T);
@@ -366,6 +356,9 @@ k3d_solver* k3d_solver_create(const k3d_params* params, int32_t device) {
     return h;  // every later call reports K3D_DEVICE_ERROR
   }
   h->blocks = step_grid_blocks(h->p.precision, h->p.pcg_threads, device);
+  // the tiled PCG serves the default CTA size of the forms with FP64 vectors
+  // (one CTA per SM); a caller's 256 or 1024 threads ask for the launch over ELL rows
+  if (h->blocks > 0 && h->vsize == 8 && h->p.pcg_threads == kSolveBlock) h->ka_smem = kachel_smem(int(h->rsize), device);
   if (h->blocks <= 0) h->err = "cannot size the cooperative grid";
   else if (h->p.pcg_bloecke > 0) h->blocks = std::min(h->blocks, h->p.pcg_bloecke);
   return h;
@@ -610,9 +603,55 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
     }
   }
 
+  // CTAs of the PCG launch per instance: in proportion to the instances' work
+  // (at least one each, largest remainders). An instance's PCG work per step
+  // grows as its points times its iteration count, and the iteration count of
+  // a 2D mesh grows as the square root of its points (the condition number
+  // grows as the mesh width squared), so the weight is points^1.5.
+  std::vector<int> nbk(ng, 1);
+  {
+    const int B = h->blocks, left = B - ng;
+    std::vector<std::pair<double, int>> rem;
+    std::vector<double> wk(ng);
+    double wsum = 0.0;
+    for (int k = 0; k < ng; ++k) {
+      const double pts = double(io[k + 1] - io[k]);
+      wk[k] = pts * std::sqrt(pts);
+      wsum += wk[k];
+    }
+    for (int k = 0; k < ng; ++k) {
+      const double share = double(left) * wk[k] / std::max(wsum, 1e-300);
+      const int whole = int(share);
+      nbk[k] += whole;
+      rem.push_back({share - double(whole), k});
+    }
+    int used = 0;
+    for (int k = 0; k < ng; ++k) used += nbk[k];
+    std::sort(rem.begin(), rem.end(), [](const auto& x, const auto& y) { return x.first > y.first || (x.first == y.first && x.second < y.second); });
+    for (size_t q = 0; used < B; ++q, ++used) nbk[rem[q % rem.size()].second] += 1;
+  }
+
+  Elemente el;
+  el.n = size_t(n);
+  el.m_p = s->membran_punkte;
+  el.b_p = s->biegung_punkte;
+  el.s_p = s_idx.data();
+  el.nt = size_t(nt);
+  el.nb = size_t(nb);
+  el.ns = size_t(ns);
+  el.off_t = off_t.data();
+  el.ent_t = ent_t.data();
+  el.off_b = off_b.data();
+  el.ent_b = ent_b.data();
+  el.off_s = off_s.data();
+  el.ent_s = ent_s.data();
+  Spalten sp;
+  spalten(el, sp);
   Pattern pat;
-  if (!build_pattern(size_t(n), np, s->membran_punkte, size_t(nt), s->biegung_punkte, size_t(nb), s_idx, pat))
-    return fail(h, K3D_BAD_ARGUMENT, "scene too large for the block pattern");
+  // tiles where they fit (k3d_plan.h); else the launch over ELL rows
+  pat.kachel = h->ka_smem > 0 && !h->p.selbstkollision && kachelplan(sp, s->x, io, nbk, R, h->p.selbstkollision != 0, h->ka_smem, kachel_kopf_bytes(), pat.plan);
+  if (pat.kachel) nbk = pat.plan.nblk;
+  if (!build_pattern(el, sp, np, pat)) return fail(h, K3D_BAD_ARGUMENT, "scene too large for the block pattern");
 
   // element constants
   std::vector<uint4> m_idx(nt), b_idx(nb);
@@ -695,8 +734,18 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
   K3D_CUDA(h, up(cv.ent_b, ent_b.data(), 4 * ent_b.size()));
   K3D_CUDA(h, up(cv.ent_s, ent_s.data(), 4 * ent_s.size()));
   K3D_CUDA(h, up(cv.cnt_v, cnt_v.data(), 4 * N));
-  K3D_CUDA(h, up(cv.row_cnt, pat.cnt.data(), 4 * N));
-  K3D_CUDA(h, up(cv.col, pat.col.data(), 4 * pat.col.size()));
+  if (pat.kachel) {
+    const Kachelplan& K = pat.plan;
+    K3D_CUDA(h, up(cv.col, K.col.data(), 4 * K.col.size()));
+    K3D_CUDA(h, up(cv.ka_blk, K.blk.data(), sizeof(KachelBlk) * K.blk.size()));
+    K3D_CUDA(h, up(cv.ka_row, K.row.data(), 4 * K.row.size()));
+    K3D_CUDA(h, up(cv.ka_halo, K.halo.data(), 4 * K.halo.size()));
+    K3D_CUDA(h, up(cv.ka_slice, K.slice.data(), sizeof(uint4) * K.slice.size()));
+    K3D_CUDA(h, up(cv.ka_lc, K.lc.data(), 2 * K.lc.size()));
+  } else {
+    K3D_CUDA(h, up(cv.row_cnt, pat.cnt.data(), 4 * N));
+    K3D_CUDA(h, up(cv.col, pat.col.data(), 4 * pat.col.size()));
+  }
   K3D_CUDA(h, up(cv.ctr_off, pat.ctr_off.data(), 4 * pat.ctr_off.size()));
   K3D_CUDA(h, up(cv.ctr, pat.ctr.data(), 4 * pat.ctr.size()));
   K3D_CUDA(h, up(cv.m_pos, m_pos.data(), 16 * T));
@@ -717,34 +766,10 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
   K3D_CUDA(h, up(cv.s_idx, s_idx.data(), 16 * S));
   K3D_CUDA(h, up(cv.s_kl, s_kl.data(), 16 * S));
 
-  // groups of the PCG launch: blocks in proportion to the instances' work
-  // (at least one each, largest remainders), points and elements per group.
-  // An instance's PCG work per step grows as its points times its iteration
-  // count, and the iteration count of a 2D mesh grows as the square root of
-  // its points (the condition number grows as the mesh width squared), so
-  // the weight is points^1.5.
+  // groups of the PCG launch: the instances' CTAs, points and elements
   {
-    const int B = h->blocks;
-    std::vector<int> nbk(ng, 1);
-    int left = B - ng;
-    std::vector<std::pair<double, int>> rem;
-    std::vector<double> wk(ng);
-    double wsum = 0.0;
-    for (int k = 0; k < ng; ++k) {
-      const double pts = double(io[k + 1] - io[k]);
-      wk[k] = pts * std::sqrt(pts);
-      wsum += wk[k];
-    }
-    for (int k = 0; k < ng; ++k) {
-      const double share = double(left) * wk[k] / std::max(wsum, 1e-300);
-      const int whole = int(share);
-      nbk[k] += whole;
-      rem.push_back({share - double(whole), k});
-    }
-    int used = 0;
-    for (int k = 0; k < ng; ++k) used += nbk[k];
-    std::sort(rem.begin(), rem.end(), [](const auto& x, const auto& y) { return x.first > y.first || (x.first == y.first && x.second < y.second); });
-    for (size_t q = 0; used < B; ++q, ++used) nbk[rem[q % rem.size()].second] += 1;
+    int B = 0;
+    for (int k : nbk) B += k;
     std::vector<Grp> grp(ng);
     std::vector<uint32_t> blk(B);
     unsigned first = 0;
@@ -939,6 +964,11 @@ static k3d_status check_sync(k3d_solver* h) {
   K3D_CUDA(h, cudaMemcpy(&ss, h->a.sync, sizeof(ss), cudaMemcpyDeviceToHost));
   if (ss.error != 0) {
     cudaMemset(&h->a.sync->error, 0, sizeof(int));
+    if (h->a.ka_blk) {  // the sequence numbers of a launch that gave up start again
+      cudaMemset(h->a.ka_wort, 0, sizeof(ulonglong2) * 6 * size_t(h->n));
+      cudaMemset(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte));
+      cudaMemset(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp));
+    }
     return fail(h, K3D_TIMEOUT, "a device barrier wait ran out of time");
   }
   return K3D_OK;

@@ -106,6 +106,7 @@ struct SelbstArgs {
   uint32_t cap_inc;
   uint32_t* inc_pos;  // per (spring << 3 | slot): its entry index, all ones for a zero weight
   void* inc_out;      // per entry: the PCG's spring product of that slot, R4
+  double* pr_c;       // the PCG direction at each spring's five points: 15 planes of cap_pairs
   int32_t* slot_of;  // damping scratch per point: its shared-memory slot, -1 between batches
   uint32_t* zahl;    // SZ_COUNT counters
   uint32_t* scan_tmp;

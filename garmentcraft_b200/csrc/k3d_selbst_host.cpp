@@ -422,6 +422,7 @@ cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap) {
   char* out = nullptr;
   if ((e = alloc(out, size_t(s.cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
   s.inc_out = out;
+  if ((e = alloc(s.pr_c, size_t(15) * cap, H.pairs)) != cudaSuccess) return e;
   return alloc(s.inc_ent, size_t(s.cap_inc), H.pairs);
 }
 
@@ -527,6 +528,8 @@ void selbst_step_args(const SelbstHost& H, StepArgs& a) {
     a.sc_w = a.sc_kf = a.sc_b0 = a.sc_b1 = nullptr;
     a.sc_bR = a.sc_wR = nullptr;
     a.sc_out = nullptr;
+    a.sc_c = nullptr;
+    a.sc_cap = 0;
     a.sc_np = 0;
     a.sc_x5 = nullptr;
     a.sc_g5 = nullptr;
@@ -545,6 +548,8 @@ void selbst_step_args(const SelbstHost& H, StepArgs& a) {
   a.sc_wR = s.pr_wR;
   a.sc_pos = s.inc_pos;
   a.sc_out = s.inc_out;
+  a.sc_c = s.pr_c;
+  a.sc_cap = s.cap_pairs;
   a.sc_x5 = s.pr_x5;
   a.sc_g5 = s.pr_g5;
   a.sc_g5R = s.pr_g5R;

@@ -134,8 +134,9 @@ static cudaError_t launch_t(const StepArgs& a, int blocks, cudaStream_t st, int&
   if (a.ev_solve0 && (e = cudaEventRecord(a.ev_solve0, st)) != cudaSuccess) return e;
   if ((e = plain(K.assemble, a, a.bplane, st)) != cudaSuccess) return e;
   launched += 1;
-  if ((e = cooperative(solve_fn_rv<R, V>(a.sc_off != nullptr, a.solve_threads), a, blocks, st)) != cudaSuccess)
-    return e;
+  e = a.ka_blk ? launch_kachel(a, st)
+               : cooperative(solve_fn_rv<R, V>(a.sc_off != nullptr, a.solve_threads), a, blocks, st);
+  if (e != cudaSuccess) return e;
   if (a.ev_solve1 && (e = cudaEventRecord(a.ev_solve1, st)) != cudaSuccess) return e;
   launched += 1;
   if (a.mode == MODE_STEP) {
@@ -149,6 +150,7 @@ static cudaError_t launch_t(const StepArgs& a, int blocks, cudaStream_t st, int&
 cudaError_t launch_pcg64(const StepArgs& a, int blocks, cudaStream_t stream) {
   StepArgs s = a;
   s.mode = MODE_SOLVE;
+  if (s.ka_blk) return launch_kachel(s, stream);
   return cooperative(solve_fn_t<double, double>(false, s.solve_threads), s, blocks, stream);
 }
 

@@ -8,7 +8,9 @@
 namespace k3d {
 
 constexpr int kBlock = 256;       // ordinary launches
-constexpr int kSolveBlock = 512;  // the persistent PCG launch's default CTA size (256 and 1024 also built)
+// the persistent PCG launch's default CTA size, and the tiled PCG's (256 and
+// 1024 are built for the launch over ELL rows)
+constexpr int kSolveBlock = 512;
 
 enum Mode : int { MODE_STEP = 0, MODE_SYSTEM = 1, MODE_OPERATOR = 2, MODE_SOLVE = 3, MODE_RESIDUAL = 4 };
 
@@ -53,6 +55,38 @@ struct Grp {
   double boden;       // convergence floor: 1e-18 of the instance's mass (implizit.rs:390-391)
   unsigned* count;    // barrier arrivals (zeroed before each launch)
   double* partials;   // kPartialsPerBlock per block of the group
+};
+
+// The tiled PCG (k3d_kachel.cu): one tile of the mesh per CTA.
+constexpr int kKachelBloecke = 160;  // most CTAs of the launch (one per SM)
+constexpr int kKachelZeilen = 4;     // most rows a thread
+constexpr int kKachelKopien = 8;     // copies of the posted sums
+// warps with rows of a CTA that posts its warps' sums: as many as keep all
+// their slabs resident (13 blocks a row)
+__host__ __device__ constexpr size_t kachel_warps(size_t rsize) { return rsize == 8 ? 6 : 8; }
+constexpr int kKachelWorte = kKachelBloecke * 8;  // posted words of a sum
+// slabs of a ring stage: two, which share a wait; one where the shared memory
+// holds few (FP64 blocks and several rows a thread)
+__host__ __device__ constexpr int kachel_griff(size_t rsize, int q) { return rsize == 8 && q > 1 ? 1 : 2; }
+constexpr int kKachelStufen = 4;     // most stages of a warp's ring of slabs
+// a slab's bytes: 32 blocks of nine values and 32 local columns
+__host__ __device__ constexpr unsigned kachel_satz(size_t rsize) { return unsigned(288 * rsize + 64); }
+__host__ __device__ constexpr size_t kachel_kopf(size_t bytes) { return (bytes + 127) & ~size_t(127); }
+// A c beside the tile in shared memory, where the registers are short
+__host__ __device__ constexpr bool kachel_ap(size_t rsize, int q) { return q > 2 || (rsize == 8 && q > 1); }
+// the tile's bytes: ns slices and halos, and A c of the slices
+__host__ __device__ constexpr size_t kachel_tile(size_t ns, size_t halos, bool ap) {
+  return (24 * (32 * ns * (ap ? 2 : 1) + halos) + 127) & ~size_t(127);
+}
+struct KachelBlk {
+  uint32_t row0, rows;    // first position (a multiple of 32) and rows of the tile
+  uint32_t halo0, halos;  // its halo's range of ka_halo
+  uint32_t platz;         // slabs of shared memory per warp
+  uint32_t stufen;        // stages of a warp's ring, at the start of its share
+  uint32_t bleibt;        // a warp's streamed slabs up to here are asked to stay in L2, the others to leave it first
+  // the posted words of a sum: this CTA's first, the group's first and how
+  // many, and whether a word is a warp's sum (else the CTA's)
+  uint32_t wort0, gruppe0, worte, einzeln;
 };
 
 struct StepArgs {
@@ -156,6 +190,25 @@ struct StepArgs {
   uint32_t* rec_flags;
   int solve_threads;  // threads per CTA of the persistent PCG launch (256, 512 or 1024)
   int pad_st;
+  // the tiled PCG (ka_blk null: the launch over ELL rows). bmat then holds
+  // slabs (kachel_satz bytes each): ctr_off, col and ka_lc are indexed by
+  // slab * 32 + lane; col is the natural column, its top bit set on the
+  // diagonal, all ones on a padding lane; ka_lc the column in the tile
+  const KachelBlk* ka_blk;
+  const uint32_t* ka_row;   // per position its point, the top bit set when another tile's halo holds it
+  const uint32_t* ka_halo;  // per halo entry its point
+  // per 32 positions: first streamed slab, streamed slabs (the first ranks),
+  // first resident slab, resident slabs (the rest); a warp's streamed slabs lie
+  // one after another, and so do its resident ones
+  const uint4* ka_slice;
+  const uint16_t* ka_lc;
+  ulonglong2* ka_wort;      // published vectors: 2 x 3 planes of n words
+  ulonglong2* ka_summe;     // posted partial sums: 2 x 2 x kKachelKopien x kKachelWorte
+  void* ka_pv;              // the preconditioner in position order: 6 planes of 32 ka_slices
+  double* ka_dv;            // dv likewise: 3 planes
+  double* sc_c;             // c of each spring's five points: 15 planes of sc_cap
+  int64_t sc_cap, ka_slices;
+  int ka_blocks, ka_q, ka_smem, ka_rsize;
   // bookkeeping
   cudaEvent_t ev_solve0, ev_solve1;  // around the PCG launch (host-side handles)
   SyncState* sync;
@@ -175,6 +228,11 @@ BuildKernels build_kernels(int precision);
 int step_grid_blocks(int precision, int threads, int device);
 // Enqueues one substep (or probe) on `stream`; `launched` = kernels enqueued.
 cudaError_t launch_step(const StepArgs& a, int precision, int blocks, cudaStream_t stream, int& launched);
+// The tiled PCG: its shared header's size, the dynamic shared memory a CTA
+// can take (0: not available here), and its launch.
+size_t kachel_kopf_bytes();
+size_t kachel_smem(int rsize, int device);
+cudaError_t launch_kachel(const StepArgs& a, cudaStream_t stream);
 // The FP64 PCG launch alone on the system built before (one pass, no release
 // test): dv (start and result), b, normals and the assembled A as in `a`.
 cudaError_t launch_pcg64(const StepArgs& a, int blocks, cudaStream_t stream);

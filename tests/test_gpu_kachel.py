@@ -1,0 +1,106 @@
+"""The tiled PCG (the default launch of the forms with FP64 vectors) against
+the launch over ELL rows, which pcg_threads=256 asks for: the same solves and
+frames at the sizes where the tiling can go wrong.
+
+Both run the same recurrences on the same blocks; only the order of the grid
+sums differs. After 20 iterations that is a few last bits times the growth of
+20 steps, far below the 1e-9 that the suite asks of well-conditioned solves.
+"""
+import numpy as np
+import pytest
+
+from garmentcraft_b200 import _abi, synth
+from garmentcraft_b200.implizit import ImplizitCg, build_scene
+from garmentcraft_b200.params import ImplizitParameter
+from garmentcraft_b200.szene import Szene
+
+pytestmark = pytest.mark.gpu
+
+FORMEN = [_abi.K3D_FP64, _abi.K3D_MIXED_STORAGE]
+TOL = 1e-9
+
+
+def laken(n, seed=3):
+    """A sheet touching its sphere, in motion, its first row pinned."""
+    m, body = synth.sheet_over_sphere(n=n, seed=seed, sdf_n=32, sdf_spacing_m=0.04, jitter_mm=200.0 / (n - 1))
+    s = build_scene(m, [body])
+    s.w[:n] = 0.0
+    rng = np.random.default_rng(seed)
+    s.x[:, 2] += 0.3 - s.x[:, 2].min() + rng.uniform(-1e-4, 1e-4, size=s.n)
+    s.v[:] = rng.normal(0.0, 0.05, size=s.v.shape)
+    s.v[:, 2] -= 0.5
+    s.param.bild_dt = 1.0 / 600.0
+    return s
+
+
+def beide(s, prec, bilder=0, **mehr):
+    """dv of a capped solve and the state after `bilder` frames, tiled and over ELL rows."""
+    aus = []
+    for threads in (0, 256):
+        q = s.copy()
+        cg = ImplizitCg(ImplizitParameter(schritte_je_bild=1, cg_max=20, cg_toleranz=1e-14, precision=prec,
+                                          pcg_threads=threads, **mehr))
+        dv0 = np.random.default_rng(1).normal(0.0, 0.01, size=q.x.shape)
+        dv, lauf = cg.loese(q, dv0)
+        for _ in range(bilder):
+            cg.bild(q)
+        aus.append((dv, lauf.iterationen, q.x, q.v, cg.statistik.kontakte))
+    return aus
+
+
+def gleich(a, b, was):
+    assert np.linalg.norm(a - b) <= TOL * np.linalg.norm(b), was
+
+
+# 2: less than a slice; 5: one ragged slice; 33: ragged CTAs; 128: 512 words, the
+# last of the natural tiles; 129: the first compact ones; 257: one row a
+# thread with a ring; 300 and 400: two and three rows a thread
+@pytest.mark.parametrize("n", [2, 5, 33, 128, 129, 257, 300, 400])
+@pytest.mark.parametrize("prec", FORMEN)
+def test_loese_und_bild(prec, n):
+    a, b = beide(laken(n), prec, bilder=1)
+    assert a[1] == b[1]
+    gleich(a[0], b[0], "dv")
+    gleich(a[2], b[2], "x")
+    gleich(a[3], b[3], "v")
+    assert a[4] == b[4]
+
+
+@pytest.mark.parametrize("bloecke", [1, 2, 7, 148])
+@pytest.mark.parametrize("prec", FORMEN)
+def test_weniger_ctas(prec, bloecke):
+    # few CTAs: several rows a thread, and natural tiles of several chunks
+    a, b = beide(laken(41), prec, bilder=1, pcg_bloecke=bloecke)
+    gleich(a[0], b[0], "dv")
+    gleich(a[2], b[2], "x")
+
+
+@pytest.mark.parametrize("prec", FORMEN)
+def test_beliebige_punktfolge(prec):
+    # points in random order: the tiles come from the positions
+    s = laken(140)
+    p = np.random.default_rng(5).permutation(s.n)  # new point i is old point p[i]
+    neu = np.empty(s.n, dtype=np.uint32)
+    neu[p] = np.arange(s.n, dtype=np.uint32)
+    kw = {f: getattr(s, f) for f in s.__dataclass_fields__}
+    for f in ("x", "v", "masse", "w", "kollisionsabstand", "reibung"):
+        kw[f] = kw[f][p].copy()
+    for f in ("abstand_punkte", "naht_punkte", "biegung_punkte", "membran_punkte", "dreiecke"):
+        kw[f] = neu[kw[f]]
+    a, b = beide(Szene(**kw), prec)
+    gleich(a[0], b[0], "dv")
+
+
+@pytest.mark.parametrize("prec", FORMEN)
+def test_stapel(prec):
+    # a batch: groups of 1 to many CTAs, each with its own sums
+    teile = []
+    for n in (3, 9, 40, 95, 17):
+        q = laken(n, seed=n)
+        teile.append(q)
+    s = Szene.verbinden(teile)
+    for bl in (0, 9):
+        a, b = beide(s, prec, bilder=1, pcg_bloecke=bl)
+        gleich(a[0], b[0], "dv")
+        gleich(a[2], b[2], "x")
+
