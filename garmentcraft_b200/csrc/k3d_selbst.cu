@@ -1471,25 +1471,13 @@ __device__ __forceinline__ uint32_t finde_schnitt(const SelbstArgs& s, uint32_t 
     if (s.sn_ke[q].y == t) return q;
   return kKein;
 }
-__device__ __forceinline__ uint32_t wurzel(uint32_t* el, uint32_t i) {
-  while (el[i] != i) {
-    el[i] = el[el[i]];
-    i = el[i];
-  }
-  return i;
-}
-__device__ __forceinline__ void vereinige(uint32_t* el, uint32_t a, uint32_t b) {
-  const uint32_t ra = wurzel(el, a), rb = wurzel(el, b);
-  if (ra != rb) el[ra > rb ? ra : rb] = ra < rb ? ra : rb;
-}
 // gebiete (selbstkollision.rs:931-1009). Linking the larger root under the
 // smaller one makes every root the smallest member of its set, so the
 // partition and the roots after the unions of the first loop do not depend
 // on their order: those run in parallel (lock-free union-find). The role
 // swaps are listed per intersection in the reference's order (counted,
 // scanned, filled); the two swap rounds, whose unions do depend on the
-// order, and the direction sums (in intersection order) run on one thread of
-// one block, in shared memory when the intersections fit.
+// order, and the direction sums (in intersection order) run in one block.
 
 // the intersections of i's region (gleich) and its role swaps (tausch), in
 // the reference's order (selbstkollision.rs:947-981)
@@ -1586,76 +1574,111 @@ __global__ void __launch_bounds__(kT) gebiete_tausch_kernel(const __grid_constan
                     [&](uint32_t j) { s.sn_tausch[q++] = make_uint2(uint32_t(i), j); });
   }
 }
-constexpr uint32_t kGebietSmem = 2048;
-constexpr size_t kGebietSmemBytes = size_t(kGebietSmem) * (2 * sizeof(uint32_t) + 3 * sizeof(double) + sizeof(double4));
-// the two swap rounds, the roots, the direction sums (one block)
-__global__ void __launch_bounds__(1024) gebiete_runden_kernel(const __grid_constant__ SelbstArgs s) {
-  extern __shared__ double gsh[];
-  __shared__ uint32_t gebiete;
-  const uint32_t n = anzahl_schnitte(s), nt = s.sn_toff[n];
+// The two swap rounds, the roots, the direction sums (one block).
+//
+// A round's partners are minima over the swaps' roots, in any order. Its
+// unions depend on their order, but all those that join nothing (nearly all:
+// there are far fewer regions than swaps) leave no trace: the block looks at
+// 1024 swaps at once from where it stands, takes the first that joins two
+// sets, and goes on behind it, which is the sequential loop's result. The
+// direction sums run root by root: each thread adds its roots' members in
+// intersection order. Parents and partners lie in shared memory up to
+// kGebietSmem intersections, in global memory beyond. On one thread over global
+// memory (over 2048 intersections) the garment's 9 k took 62 ms.
+constexpr uint32_t kGebietSmem = 24576;
+constexpr size_t kGebietSmemBytes = size_t(kGebietSmem) * 2 * sizeof(uint32_t);
+constexpr uint32_t kGebietT = 1024;
+__global__ void __launch_bounds__(kGebietT) gebiete_runden_kernel(const __grid_constant__ SelbstArgs s) {
+  extern __shared__ uint32_t gsh[];
+  __shared__ uint4 wurzeln[kGebietT / 4];
+  __shared__ uint32_t gebiete, erste;
+  const uint32_t n = anzahl_schnitte(s), nt = s.sn_toff[n], tid = threadIdx.x;
   const bool sm = n <= kGebietSmem;
-  double4* g = reinterpret_cast<double4*>(gsh);
-  double* summe = gsh + 4 * kGebietSmem;
-  uint32_t* el = sm ? reinterpret_cast<uint32_t*>(summe + 3 * kGebietSmem) : s.sn_eltern;
-  uint32_t* partner = sm ? el + kGebietSmem : s.sn_partner;
-  if (threadIdx.x == 0) gebiete = 0;
+  uint32_t* el = sm ? gsh : s.sn_eltern;
+  uint32_t* partner = sm ? gsh + kGebietSmem : s.sn_partner;
+  if (tid == 0) gebiete = 0;
   if (sm)
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      el[i] = s.sn_eltern[i];
-      g[i] = s.sn_g[i];
-      summe[3 * i] = summe[3 * i + 1] = summe[3 * i + 2] = 0.0;
-    }
+    for (uint32_t i = tid; i < n; i += kGebietT) el[i] = s.sn_eltern[i];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int runde = 0; runde < 2; ++runde) {
-      for (uint32_t i = 0; i < n; ++i) partner[i] = kKein;
-      for (uint32_t q = 0; q < nt; ++q) {
+  for (int runde = 0; runde < 2; ++runde) {
+    // straight to the roots (a parent is read while another thread shortens
+    // its path: either value leads to the same root)
+    for (uint32_t i = tid; i < n; i += kGebietT) {
+      *reinterpret_cast<volatile uint32_t*>(&el[i]) = wurzel_lesen(el, i);
+      partner[i] = kKein;
+    }
+    __syncthreads();
+    for (uint32_t q = tid; q < nt; q += kGebietT) {
+      const uint2 ij = s.sn_tausch[q];
+      const uint32_t ri = wurzel_lesen(el, ij.x), rj = wurzel_lesen(el, ij.y);
+      atomicMin(&partner[ri], rj);
+      atomicMin(&partner[rj], ri);
+    }
+    __syncthreads();
+    for (uint32_t q0 = 0; q0 < nt;) {
+      if (tid == 0) erste = kKein;
+      __syncthreads();
+      const uint32_t q = q0 + tid;
+      uint32_t ra = 0, rb = 0;
+      if (q < nt) {
         const uint2 ij = s.sn_tausch[q];
-        const uint32_t ri = wurzel(el, ij.x), rj = wurzel(el, ij.y);
-        if (rj < partner[ri]) partner[ri] = rj;
-        if (ri < partner[rj]) partner[rj] = ri;
+        const uint32_t p = *reinterpret_cast<volatile uint32_t*>(&partner[wurzel_lesen(el, ij.y)]);
+        if (p != kKein) {
+          ra = wurzel_lesen(el, ij.x);
+          rb = wurzel_lesen(el, p);
+          if (ra != rb) atomicMin(&erste, q);
+        }
       }
-      for (uint32_t q = 0; q < nt; ++q) {
-        const uint2 ij = s.sn_tausch[q];
-        const uint32_t rj = wurzel(el, ij.y);
-        if (partner[rj] != kKein) vereinige(el, ij.x, partner[rj]);
-      }
+      __syncthreads();
+      const uint32_t e = erste;
+      if (q == e) *reinterpret_cast<volatile uint32_t*>(&el[ra > rb ? ra : rb]) = ra < rb ? ra : rb;
+      q0 = e == kKein ? q0 + kGebietT : e + 1;
+      __syncthreads();
     }
   }
-  __syncthreads();
   uint32_t eigene = 0;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+  for (uint32_t i = tid; i < n; i += kGebietT) {
     const uint32_t r = wurzel_lesen(el, i);
     s.sn_wurzel[i] = r;
     if (r == i) ++eigene;
-    if (!sm) s.sn_summe[i] = make_double4(0, 0, 0, 0);
+    s.sn_summe[i] = make_double4(0, 0, 0, 0);
   }
   if (eigene) atomicAdd(&gebiete, eigene);
   __syncthreads();
-  if (threadIdx.x == 0) {  // the sums in intersection order, as the reference adds them
-    for (uint32_t i = 0; i < n; ++i) {
-      const uint32_t r = s.sn_wurzel[i];
-      if (sm) {
-        const double4 gi = g[i];
-        summe[3 * r] += gi.x * gi.w;
-        summe[3 * r + 1] += gi.y * gi.w;
-        summe[3 * r + 2] += gi.z * gi.w;
-      } else {
-        const double4 gi = s.sn_g[i];
-        double4& m = s.sn_summe[r];
+  // the sums in intersection order, as the reference adds them: thread t the
+  // roots t, t + 1024, ...
+  uint32_t cur = kKein;
+  D3 m = d3(0.0, 0.0, 0.0);
+  for (uint32_t i0 = 0; i0 < n; i0 += kGebietT) {
+    reinterpret_cast<uint32_t*>(wurzeln)[tid] = i0 + tid < n ? s.sn_wurzel[i0 + tid] : kKein;
+    __syncthreads();
+    for (uint32_t j = 0; j < kGebietT / 4 && i0 + 4 * j < n; ++j) {
+      const uint4 w = wurzeln[j];
+      const uint32_t r4[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t r = r4[k];
+        if (r == kKein || r % kGebietT != tid) continue;
+        if (r != cur) {
+          if (cur != kKein) s.sn_summe[cur] = make_double4(m.x, m.y, m.z, 0.0);
+          cur = r;
+          const double4 z = s.sn_summe[r];
+          m = d3(z.x, z.y, z.z);
+        }
+        const double4 gi = s.sn_g[i0 + 4 * j + k];
         m.x += gi.x * gi.w;
         m.y += gi.y * gi.w;
         m.z += gi.z * gi.w;
       }
     }
-    s.zahl[SZ_GEBIETE] = gebiete;
+    __syncthreads();
   }
+  if (cur != kKein) s.sn_summe[cur] = make_double4(m.x, m.y, m.z, 0.0);
+  if (tid == 0) s.zahl[SZ_GEBIETE] = gebiete;
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint32_t r = s.sn_wurzel[i];
-    const D3 m = sm ? d3(summe[3 * r], summe[3 * r + 1], summe[3 * r + 2])
-                    : d3(s.sn_summe[r].x, s.sn_summe[r].y, s.sn_summe[r].z);
-    const D3 u = einheit(m);
+  for (uint32_t i = tid; i < n; i += kGebietT) {
+    const double4 z = s.sn_summe[s.sn_wurzel[i]];
+    const D3 u = einheit(d3(z.x, z.y, z.z));
     s.sn_g[i] = make_double4(u.x, u.y, u.z, s.sn_g[i].w);
   }
 }
@@ -2437,7 +2460,7 @@ cudaError_t selbst_paare_und_federn(const SelbstArgs& s, uint32_t n_aktiv_p, uin
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = scan(s.sn_toff, int64_t(n_s) + 1, s.sn_scan_tmp, nullptr, st)) != cudaSuccess) return e;
   gebiete_tausch_kernel<<<grid_for(n_s), kT, 0, st>>>(s);
-  gebiete_runden_kernel<<<1, 1024, kGebietSmemBytes, st>>>(s);
+  gebiete_runden_kernel<<<1, kGebietT, kGebietSmemBytes, st>>>(s);
   klemm_kernel<<<grid_for(ns), kT, 0, st>>>(s);
   folge_kernel<<<grid_for(s.nd), kT, 0, st>>>(s);
   if (s.rsize == 4)
