@@ -14,6 +14,7 @@
 namespace k3d {
 namespace netz {
 
+constexpr int kEben = 5;
 struct Dev {
   int64_t n, nd;
   double suchtiefe;
@@ -23,6 +24,8 @@ struct Dev {
   const uint4* nb;  // neighbour across edge k (the triangle itself at an open edge)
   double4* pn;      // angle-weighted point normal
   double4* kg;      // bounding sphere: centre, radius
+  float4* ef;       // its own frame in FP32, kEben per triangle (flaechen_kernel)
+  uint2* ez;        // first cell of the triangle's range: (x | y << 16, z)
   double* wk;       // corner angles, 3 per triangle
   double* vt;       // volume term per triangle
   const uint32_t *pi_off, *pi_ent;
@@ -32,6 +35,7 @@ struct Dev {
   int32_t zx, zy, zz;
   uint32_t *anf, *ein, *cur;
   uint32_t cap;
+  float weit;  // no coordinate of the mesh is farther from zero
   uint32_t *pg_anf, *pg_ein;  // point grid on the same cells (Z + 1 starts; N entries, ascending per cell)
 };
 
