@@ -34,11 +34,14 @@ void spalten(const Elemente& E, Spalten& S) {
 
 namespace {
 
-// Bytes of slabs that stay in the 126 MB L2 beside the vectors and the words.
-// Measured, cycles an iteration without -> with the rule: 202 k points, FP32
-// blocks (118 MB) 74 k -> 63 k; 160 k, FP64 (219 MB) 100 k -> 87 k; 205 k points of
-// the garment, FP32 blocks 78 k -> 69 k.
-constexpr size_t kKachelL2 = size_t(64) << 20;
+// Bytes of streamed slabs that are asked to stay in L2 where there are more of
+// them. Measured, thousand cycles an iteration with 100 (no rule), 64, 40, 24,
+// 16 and 8 MB: 160 k points, FP32 blocks (65 MB streamed) 49.6, 49.3, 47.9,
+// 42.1, 42.9, 45.0; 160 k, FP64 (146 MB) 94.8, -, 77.9, 74.0, 72.5, 72.0;
+// 205 k of a garment, FP32 blocks -, 62.2, 54.7, 52.1, 52.2, 52.5; 90 k, FP64
+// (81 MB) 48.2, -, 43.4, 43.3, 44.0, 41.3; up to 55 MB no difference. So little:
+// each half of the L2 keeps its own copy of what its SMs read.
+constexpr size_t kKachelL2 = size_t(24) << 20;
 
 // Splits the points idx[lo, hi) into nb parts of whole slices (the last one
 // may be ragged), in the order of the bisection, across the longest side of
@@ -247,9 +250,9 @@ bool kachelplan(const Spalten& S, const double* x, const std::vector<int64_t>& i
     }
   }
   if (P.slabs * 32 >= (size_t(1) << 32)) return false;
-  // What an iteration streams comes round again in the same order, so beyond
-  // the L2's size each slab is evicted before its next turn. A part is then
-  // asked to stay and the rest to leave first.
+  // What an iteration streams comes round again in the same order, so where the
+  // L2 cannot keep it all each slab is evicted before its next turn. A part is
+  // then asked to stay and the rest to leave first.
   {
     size_t alle = 0;
     for (const uint4& s : P.slice) alle += s.y;
