@@ -247,7 +247,7 @@ static void carve(k3d_solver* h, Arena& A, size_t N, size_t T, size_t B, size_t 
     a.ka_halo = cv.ka_halo = A.take<uint32_t>(K.halo.size());
     a.ka_slice = cv.ka_slice = A.take<uint4>(K.slice.size());
     a.ka_lc = cv.ka_lc = A.take<uint16_t>(nbs);
-    a.ka_wort = A.take<ulonglong2>(6 * N);
+    a.ka_wort = A.take<ulonglong2>((h->p.selbstkollision ? 12 : 6) * N);
     a.ka_pv = A.take<char>(6 * 32 * K.slice.size() * R);
     a.ka_dv = A.take<double>(3 * 32 * K.slice.size());
     a.ka_summe = A.take<ulonglong2>(4 * size_t(kKachelKopien) * size_t(kKachelWorte));
@@ -358,7 +358,7 @@ k3d_solver* k3d_solver_create(const k3d_params* params, int32_t device) {
   h->blocks = step_grid_blocks(h->p.precision, h->p.pcg_threads, device);
   // the tiled PCG serves the default CTA size of the forms with FP64 vectors
   // (one CTA per SM); a caller's 256 or 1024 threads ask for the launch over ELL rows
-  if (h->blocks > 0 && h->vsize == 8 && h->p.pcg_threads == kSolveBlock) h->ka_smem = kachel_smem(int(h->rsize), device);
+  if (h->blocks > 0 && h->vsize == 8 && h->p.pcg_threads == kSolveBlock) h->ka_smem = kachel_smem(device);
   if (h->blocks <= 0) h->err = "cannot size the cooperative grid";
   else if (h->p.pcg_bloecke > 0) h->blocks = std::min(h->blocks, h->p.pcg_bloecke);
   return h;
@@ -649,7 +649,9 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
   spalten(el, sp);
   Pattern pat;
   // tiles where they fit (k3d_plan.h); else the launch over ELL rows
-  pat.kachel = h->ka_smem > 0 && !h->p.selbstkollision && kachelplan(sp, s->x, io, nbk, R, h->p.selbstkollision != 0, h->ka_smem, kachel_kopf_bytes(), pat.plan);
+  const bool federn = h->p.selbstkollision != 0;
+  pat.kachel = h->ka_smem > 0 && kachelplan(sp, s->x, io, nbk, R, federn, h->ka_smem, kachel_kopf_bytes(), pat.plan) &&
+               kachel_bereit(int(R), federn, pat.plan.q, h->ka_smem);
   if (pat.kachel) nbk = pat.plan.nblk;
   if (!build_pattern(el, sp, np, pat)) return fail(h, K3D_BAD_ARGUMENT, "scene too large for the block pattern");
 
@@ -857,6 +859,7 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
       return fail(h, K3D_BAD_ARGUMENT, "scene too large for the self-collision stage");
     K3D_CUDA(h, selbst_upload(h->sc, s, h->p.selbst_zusatzdicke, h->p.selbst_steifigkeit, int(R), a.x, a.v, cv.masse,
                               cv.w, cv.reib, st));
+    if (pat.kachel) K3D_CUDA(h, selbst_grow_zeilen(h->sc, uint32_t(4 * n + 1024)));
   }
 
   a.n = n;
@@ -965,7 +968,7 @@ static k3d_status check_sync(k3d_solver* h) {
   if (ss.error != 0) {
     cudaMemset(&h->a.sync->error, 0, sizeof(int));
     if (h->a.ka_blk) {  // the sequence numbers of a launch that gave up start again
-      cudaMemset(h->a.ka_wort, 0, sizeof(ulonglong2) * 6 * size_t(h->n));
+      cudaMemset(h->a.ka_wort, 0, sizeof(ulonglong2) * (h->p.selbstkollision ? 12 : 6) * size_t(h->n));
       cudaMemset(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte));
       cudaMemset(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp));
     }

@@ -13,7 +13,7 @@
 //  * the blocks lie in slabs (32 rows of one warp x one rank, with their
 //    columns). As many slabs as fit stay in shared memory for the whole
 //    launch; the others pass through a ring of bulk copies that each warp
-//    keeps full by itself, across the barriers of the iteration;
+//    keeps full by itself, its first copies on their way before the sum is in;
 //  * halo values and the CTAs' partial sums travel as words that carry their
 //    own sequence number beside 32 bits of payload: a reader polls the datum
 //    itself, so an exchange costs one store and one load latency, without
@@ -31,6 +31,10 @@
 // product at 30 cycles a slab (23 shared-memory wavefronts, 18 of the
 // conversion unit); beyond, the slabs that do not fit on the SMs, at 9-10 TB/s
 // from L2.
+// Self-collision springs come as merged rows of blocks (federzeilen): with the
+// launch over ELL rows, which forms each spring's products and sums them by
+// point, 205 k points with 63 k springs, 3051 iterations, took 217 ms, here
+// 117 ms; two layers of 3 k points, 907 iterations in ten solves, 30 ms and 16.
 // Sums are deterministic: a fixed tree per CTA, then the CTAs' partials in
 // CTA order in every CTA. Every wait is bounded (kBarrierLimitNs): it records
 // K3D_TIMEOUT, the warps wait for their copies in flight, and all return.
@@ -43,7 +47,7 @@ constexpr int kNT = kSolveBlock;
 constexpr int kNW = kNT / 32;
 
 // A slab: 32 blocks as two 4-vectors and a scalar per lane, then the lanes'
-// local columns (byte offsets).
+// local columns.
 template <typename R>
 struct Satz {
   static constexpr unsigned v = 128 * sizeof(R), w = 256 * sizeof(R), spalte = 288 * sizeof(R);
@@ -61,6 +65,7 @@ struct KSh {
   Grp g;
   KachelBlk b;
   unsigned bidx;
+  unsigned federn;  // rows of springs of this CTA
   int err;
 };
 
@@ -122,11 +127,10 @@ __device__ __forceinline__ ulonglong2* summe(const StepArgs& a, uint32_t seq, un
   return a.ka_summe + (((size_t(seq & 1u) * 2 + k) * kKachelKopien) + c) * kKachelWorte;
 }
 // Posts this CTA's part of NV sums under the sequence number `seq`, its
-// warps' sums or their sum in warp order; with `fest` (CTA sums only) the
-// CTA's earlier global writes are visible to who has waited. Every warp of the CTA has come
-// this far when it returns.
+// warps' sums or their sum in warp order. Every warp of the CTA has come this
+// far when it returns.
 template <int NV>
-__device__ __forceinline__ void melden(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq, bool fest = false) {
+__device__ __forceinline__ void melden(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool einzeln = sh.b.einzeln != 0;
 #pragma unroll
@@ -142,8 +146,6 @@ __device__ __forceinline__ void melden(const StepArgs& a, KSh& sh, double (&v)[N
   }
   __syncthreads();
   if (!einzeln && warp == 0) {
-    if (fest && lane == 0) fence_acq_rel();
-    __syncwarp();
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       double x = 0.0;
@@ -167,7 +169,7 @@ __device__ __forceinline__ void vorab(const StepArgs& a, const KSh& sh, Vorab& v
     v.da = ld_wort(summe(a, seq, sh.bidx % kKachelKopien, 0) + sh.b.gruppe0 + threadIdx.x, seq, v.v);
 }
 template <int NV>
-__device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq, bool fest = false,
+__device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq,
                                         Vorab vor = Vorab()) {
   const unsigned nb = sh.b.worte, lane = threadIdx.x & 31;
   const bool einzeln = sh.b.einzeln != 0;
@@ -177,7 +179,6 @@ __device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[
     for (int k = 0; k < NV; ++k)
       sh.arr[k][i] = k == 0 && vor.da ? vor.v
                                       : hol_wort(a, sh, summe(a, seq, sh.bidx % kKachelKopien, k) + sh.b.gruppe0 + threadIdx.x, seq);
-    if (fest) fence_acq_rel();
   }
   __syncthreads();
   if (*reinterpret_cast<volatile int*>(&sh.err) != 0) return false;
@@ -367,111 +368,53 @@ __device__ __forceinline__ D3 s_filter(D3 n, D3 x) {
   return d3(x.x - n.x * d, x.y - n.y * d, x.z - n.z * d);
 }
 
-// Self-collision springs at point i applied to dv (start residual, release
-// test), with the operator-precision blocks.
-template <typename R>
-__device__ __noinline__ D3 federn_dv(const StepArgs& a, int64_t i) {
-  const R4<R>* bR = static_cast<const R4<R>*>(a.sc_bR);
-  const R4<R>* wR = static_cast<const R4<R>*>(a.sc_wR);
-  const R* g5R = static_cast<const R*>(a.sc_g5R);
-  D3 o = d3(0.0, 0.0, 0.0);
-  const D3 pi = ld3(a.dv, uint32_t(i));
-  for (uint32_t e = a.sc_off[i]; e < a.sc_off[i + 1]; ++e) {
-    const uint32_t ent = a.sc_ent[e], q = ent >> 3, k = ent & 7u;
-    const uint4 id = a.sc_idx[q];
-    const R4<R> w4 = wR[q];
-    const double g[5] = {double(w4.x), double(w4.y), double(w4.z), double(w4.w), double(g5R[q])};
-    const uint32_t ix[5] = {id.x, id.y, id.z, id.w, a.sc_x5[q]};
-    const double gk = k == 0 ? g[0] : k == 1 ? g[1] : k == 2 ? g[2] : k == 3 ? g[3] : g[4];
-    double sx = 0.0, sy = 0.0, sz = 0.0;
+// The self-collision springs' part of a product, t = F w, in their merged rows
+// (SelbstArgs::sf_*). The points in contact lie in few tiles, so the rows are
+// spread over every CTA: eight lanes a row take its blocks against the
+// published words of its columns and publish t in turn, and the point's own
+// thread adds it after the tile's product. What bounds it is latency, so the
+// rows' heads lie in shared memory (kopf: starts, blocks, columns) and the
+// blocks travel with the words.
+__device__ __forceinline__ void federzeilen(const StepArgs& a, KSh& sh, const uint32_t* kopf, uint32_t ep) {
+  const unsigned l = threadIdx.x & 7;
+  const ulonglong2* wort = a.ka_wort + size_t(ep & 1u) * 3 * size_t(a.n);
+  ulonglong2* aus = a.ka_wort + (2 + size_t(ep & 1u)) * 3 * size_t(a.n);
+  const size_t cap = size_t(a.sf_cap);
+#pragma unroll 1
+  for (unsigned g = threadIdx.x >> 3; __any_sync(0xffffffffu, g < sh.federn); g += kNT / 8) {
+    const bool nah = g < kFederZeilen;
+    unsigned anf = 0, m = 0;
+    if (g < sh.federn) {
+      anf = nah ? kopf[g] : a.sf_anf[g * sh.g.nblk + sh.bidx];
+      m = nah ? kopf[kFederZeilen + g] : a.sf_anz[g * sh.g.nblk + sh.bidx];
+    }
+    double x = 0.0, y = 0.0, z = 0.0;
+    uint32_t i = 0;
+#pragma unroll 1
+    for (unsigned e = l; e < m; e += 8) {
+      const uint32_t j =
+          nah && e < kFederSpalten ? kopf[2 * kFederZeilen + kFederSpalten * g + e] : a.sf_spalte[anf + e];
+      const double* b = a.sf_block + anf + e;
+      const double bxx = b[0], byy = b[cap], bzz = b[2 * cap], bxy = b[3 * cap], bxz = b[4 * cap], byz = b[5 * cap];
+      const D3 w = hol_wort3(a, sh, wort + j, ep);
+      x += bxx * w.x + bxy * w.y + bxz * w.z;
+      y += bxy * w.x + byy * w.y + byz * w.z;
+      z += bxz * w.x + byz * w.y + bzz * w.z;
+      if (e < 8) i = j;
+    }
+    __syncwarp();
 #pragma unroll
-    for (int r = 0; r < 5; ++r)
-      if ((gk > 0.0 && g[r] < 0.0) || (gk < 0.0 && g[r] > 0.0)) {
-        const double om = -gk * g[r];
-        const D3 pr = ld3(a.dv, ix[r]);
-        sx += om * (pi.x - pr.x);
-        sy += om * (pi.y - pr.y);
-        sz += om * (pi.z - pr.z);
-      }
-    const R4<R> b0 = bR[2 * q], b1 = bR[2 * q + 1];
-    o.x += double(b0.x) * sx + double(b0.w) * sy + double(b1.x) * sz;
-    o.y += double(b0.w) * sx + double(b0.y) * sy + double(b1.y) * sz;
-    o.z += double(b1.x) * sx + double(b1.y) * sy + double(b0.z) * sz;
+    for (int o = 4; o > 0; o >>= 1) {
+      x += __shfl_xor_sync(0xffffffffu, x, o);
+      y += __shfl_xor_sync(0xffffffffu, y, o);
+      z += __shfl_xor_sync(0xffffffffu, z, o);
+    }
+    i = __shfl_sync(0xffffffffu, i, 0, 8);  // the diagonal's column
+    if (m > 0 && l < 3) st_wort(aus + l * size_t(a.n) + i, l == 0 ? x : l == 1 ? y : z, ep);
   }
-  return o;
 }
 
-// The springs' share of an iteration, spring by spring over the whole grid
-// (implizit.rs:214-220): each spring keeps c of its five points (sc_c), takes
-// w from the published words, and leaves each slot's product in its entry;
-// the points add their entries in list order after the next grid sum. Returns
-// this thread's part of c.A c.
-template <typename R>
-__device__ __forceinline__ double federn_c(const StepArgs& a, KSh& sh, const ulonglong2* wort, uint32_t ep, double beta,
-                                           bool erste) {
-  const R4<R>* bR = static_cast<const R4<R>*>(a.sc_bR);
-  const R4<R>* wR = static_cast<const R4<R>*>(a.sc_wR);
-  const R* g5R = static_cast<const R*>(a.sc_g5R);
-  R4<double>* out = static_cast<R4<double>*>(a.sc_out);
-  double ca = 0.0;
-  const int64_t nth = int64_t(sh.g.nblk) * kNT, np = int64_t(a.sc_np);
-  for (int64_t q = nth - 1 - (int64_t(sh.bidx) * kNT + threadIdx.x); q < np; q += nth) {
-    const uint4 id = a.sc_idx[q];
-    const R4<R> w4 = wR[q];
-    const double g[5] = {double(w4.x), double(w4.y), double(w4.z), double(w4.w), double(g5R[q])};
-    const uint32_t ix[5] = {id.x, id.y, id.z, id.w, a.sc_x5[q]};
-    const R4<R> b0 = bR[2 * q], b1 = bR[2 * q + 1];
-    const uint4 pos4 = *reinterpret_cast<const uint4*>(&a.sc_pos[8 * q]);
-    const uint32_t pos[5] = {pos4.x, pos4.y, pos4.z, pos4.w, a.sc_pos[8 * q + 4]};
-    // every load first; a point of weight zero takes no part and may not be
-    // published
-    D3 c[5], w[5];
-    bool da[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      c[r] = w[r] = d3(0.0, 0.0, 0.0);
-      da[r] = true;
-      if (g[r] == 0.0) continue;
-      if (!erste) {
-        const double* cc = a.sc_c + size_t(3 * r) * size_t(a.sc_cap) + q;
-        c[r] = d3(cc[0], cc[a.sc_cap], cc[2 * size_t(a.sc_cap)]);
-      }
-      da[r] = ld_wort3(wort + ix[r], a.n, ep, w[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      if (g[r] == 0.0) continue;
-      if (!da[r]) w[r] = hol_wort3(a, sh, wort + ix[r], ep);
-      c[r] = d3(fmar(beta, c[r].x, w[r].x), fmar(beta, c[r].y, w[r].y), fmar(beta, c[r].z, w[r].z));
-      double* cc = a.sc_c + size_t(3 * r) * size_t(a.sc_cap) + q;
-      cc[0] = c[r].x;
-      cc[a.sc_cap] = c[r].y;
-      cc[2 * size_t(a.sc_cap)] = c[r].z;
-    }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const uint32_t e = pos[k];
-      if (e == 0xffffffffu) continue;
-      double sx = 0.0, sy = 0.0, sz = 0.0;
-#pragma unroll
-      for (int r = 0; r < 5; ++r)
-        if ((g[k] > 0.0 && g[r] < 0.0) || (g[k] < 0.0 && g[r] > 0.0)) {
-          const double om = -g[k] * g[r];
-          sx += om * (c[k].x - c[r].x);
-          sy += om * (c[k].y - c[r].y);
-          sz += om * (c[k].z - c[r].z);
-        }
-      const double tx = double(b0.x) * sx + double(b0.w) * sy + double(b1.x) * sz;
-      const double ty = double(b0.w) * sx + double(b0.y) * sy + double(b1.y) * sz;
-      const double tz = double(b1.x) * sx + double(b1.y) * sy + double(b0.z) * sz;
-      out[e] = {tx, ty, tz, 0.0};
-      ca += c[k].x * tx + c[k].y * ty + c[k].z * tz;
-    }
-  }
-  return ca;
-}
-
-enum : unsigned { kZeile = 1u, kFrei = 2u, kGehalten = 4u, kGrenze = 8u };
+enum : unsigned { kZeile = 1u, kFrei = 2u, kGehalten = 4u, kGrenze = 8u, kFedern = 16u };
 
 // Q rows a thread (slices of 32 rows: warp, warp + 16, ...).
 template <typename R, bool SC, int Q>
@@ -487,6 +430,10 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     sh.g = a.grp[a.blk_grp[blockIdx.x]];
     sh.b = a.ka_blk[blockIdx.x];
     sh.bidx = blockIdx.x - sh.g.first_blk;
+    if (SC) {
+      const unsigned z = *a.sf_zahl;
+      sh.federn = z > sh.bidx ? (z - sh.bidx + sh.g.nblk - 1) / sh.g.nblk : 0u;
+    }
   }
   if (lane == 0) {
     for (int s = 0; s <= kKachelStufen; ++s) bar_init(&sh.bar[warp][s]);
@@ -524,8 +471,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       const uint32_t z = a.ka_row[sh.b.row0 + r];
       pt[q] = z & 0x7fffffffu;
       fl[q] = kZeile | (a.frei[pt[q]] ? kFrei : 0u) | (z >> 31 ? kGrenze : 0u);
-      // the springs of other CTAs may read this point
-      if (SC && a.sc_off[pt[q]] != a.sc_off[pt[q] + 1]) fl[q] |= kGrenze;
+      if (SC && a.sc_off[pt[q]] != a.sc_off[pt[q] + 1]) fl[q] |= kGrenze | kFedern;
     }
   }
   // the warp's share of the shared memory behind the tile: its ring, then its
@@ -533,7 +479,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
   {
     g.stufen = sh.b.stufen;
     g.bleibt = sh.b.bleibt;
-    g.ring = unsigned(kachel_kopf(sizeof(KSh)) + kachel_tile(ns, halos, kAp)) +
+    g.ring = unsigned(kachel_kopf(sizeof(KSh)) + kachel_tile(sizeof(R), ns, halos, kAp, SC)) +
              unsigned(warp) * sh.b.platz * Satz<R>::bytes;
     g.fest = g.ring + g.stufen * U * Satz<R>::bytes;
     unsigned long long* bar = sh.bar[warp];
@@ -602,6 +548,22 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     return d3(p[0], p[1], p[2]);
   };
   double* ap_s = halo + 3 * halos;
+  double* f_s = ap_s + (kAp ? 3 * 32 * ns : 0);  // with FP64 blocks the springs' part of A c
+  uint32_t* fkopf = reinterpret_cast<uint32_t*>(g_roh + kachel_kopf(sizeof(KSh)) +
+                                                kachel_vektoren(sizeof(R), ns, halos, kAp, SC));
+  if (SC) {  // heads of the springs' rows
+    const unsigned nf = sh.federn < kFederZeilen ? sh.federn : kFederZeilen;
+    for (unsigned t = threadIdx.x; t < nf * kFederSpalten; t += kNT) {
+      const unsigned z = t / kFederSpalten, e = t % kFederSpalten, k = z * sh.g.nblk + sh.bidx;
+      const uint32_t anf = a.sf_anf[k], m = a.sf_anz[k];
+      if (e == 0) {
+        fkopf[z] = anf;
+        fkopf[kFederZeilen + z] = m;
+      }
+      if (e < m) fkopf[2 * kFederZeilen + t] = a.sf_spalte[anf + e];
+    }
+    __syncthreads();
+  }
   auto ap_lesen = [&](int q) -> D3 {
     if (!kAp) return d3(ap[kAp ? 0 : q][0], ap[kAp ? 0 : q][1], ap[kAp ? 0 : q][2]);
     const double* p = ap_s + 3 * (32 * (warp + kNW * q) + lane);
@@ -621,8 +583,27 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       halo[3 * t + 2] = v.z;
     }
   };
-  // the tile takes dv, its halo too; with SC dv is in place in memory and
-  // visible to every CTA
+  // o += the springs' product, of the vector published under e: t of w, or
+  // (FP64 blocks) of c = w + beta c_prev by t + beta times its last value
+  auto federn = [&](uint32_t e, double bt, bool neu) {
+    const ulonglong2* p = a.ka_wort + (2 + size_t(e & 1u)) * 3 * size_t(a.n);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!(fl[q] & kFedern)) continue;
+      D3 t = hol_wort3(a, sh, p + pt[q], e);
+      if (!kRec && !neu) {
+        double* f = f_s + 3 * (32 * (warp + kNW * q) + lane);
+        if (bt != 0.0) t = d3(fmar(bt, f[0], t.x), fmar(bt, f[1], t.y), fmar(bt, f[2], t.z));
+        f[0] = t.x;
+        f[1] = t.y;
+        f[2] = t.z;
+      }
+      o[q][0] += t.x;
+      o[q][1] += t.y;
+      o[q][2] += t.z;
+    }
+  };
+  // the tile takes dv, its halo too; so do the springs' rows
   auto dv_auslegen = [&]() -> bool {
     ++ep;
 #pragma unroll
@@ -633,13 +614,8 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       ausgeben(q, d);
       eigen(q, d);
     }
-    if (SC) {
-      double null[1] = {0.0};
-      ++seq;
-      melden<1>(a, sh, null, seq, true);
-      if (!sammeln<1>(a, sh, null, seq, true)) return false;
-    }
     halo_holen();
+    if (SC) federzeilen(a, sh, fkopf, ep);
     __syncthreads();
     return *reinterpret_cast<volatile int*>(&sh.err) == 0;
   };
@@ -681,10 +657,10 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         dv[q % (kDv ? Q : 1)][2] = d.z;
       }
       if (!kDv) dv_schreiben(q, d);
-      if (SC) st3(a.dv, pt[q], d);
     }
     if (!(gut = dv_auslegen())) break;
     produkt<R, Q>(a, sh, g, strom, fest, o);
+    if (SC) federn(ep, 0.0, true);
     double red[2] = {0.0, 0.0};
     ++ep;
 #pragma unroll
@@ -693,7 +669,6 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       if (fl[q] & kFrei) {
         const D3 b = ld3(a.b, pt[q]);
         D3 ad = d3(o[q][0], o[q][1], o[q][2]);
-        if (SC) ad = ad + federn_dv<R>(a, pt[q]);
         const D3 n = normale(q);
         D3 rd = b - ad;
         rd = rd - n * dot(rd, n);
@@ -744,6 +719,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       Vorab vor;
       if (kRec) {
         halo_holen();
+        if (SC) federzeilen(a, sh, fkopf, ep);
         __syncthreads();
         if (*reinterpret_cast<volatile int*>(&sh.err) != 0) {
           gut = false;
@@ -751,18 +727,20 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         }
         vorab(a, sh, vor, seq);  // its latency passes under the product
         produkt<R, Q>(a, sh, g, strom, fest, o);
-      } else if (threadIdx.x < halos) {  // the first chunk of the halo while the sum travels
-        da = ld_wort3(wort() + halo_pt[threadIdx.x], a.n, ep, hw);
+        if (SC) federn(ep, 0.0, true);
+      } else {  // the first chunk of the halo and the springs while the sum travels
+        if (threadIdx.x < halos) da = ld_wort3(wort() + halo_pt[threadIdx.x], a.n, ep, hw);
+        if (SC) federzeilen(a, sh, fkopf, ep);
       }
       if (erste) {
         double s[2];
-        if (!(gut = sammeln<2>(a, sh, s, seq, false, vor))) break;
+        if (!(gut = sammeln<2>(a, sh, s, seq, vor))) break;
         delta = s[0];
         bb = s[1];
         ziel = fmax(a.tol * a.tol * fmax(bb, delta), sh.g.boden);
       } else {
         double s[1];
-        if (!(gut = sammeln<1>(a, sh, s, seq, false, vor))) break;
+        if (!(gut = sammeln<1>(a, sh, s, seq, vor))) break;
         beta = s[0] / delta;
         delta = s[0];
         ++it;
@@ -788,6 +766,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
           break;
         }
         produkt<R, Q>(a, sh, g, strom, fest, o);
+        if (SC) federn(ep, beta, false);
       }
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
@@ -811,10 +790,9 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         ap_setzen(q, s);
         ca[0] += c.x * s.x + c.y * s.y + c.z * s.z;
       }
-      if (SC) ca[0] += federn_c<R>(a, sh, wort(), ep, beta, erste);
       erste = false;
       ++seq;
-      melden<1>(a, sh, ca, seq, SC);
+      melden<1>(a, sh, ca, seq);
       // the update's loads travel with the sum
       R p2[kNah ? 1 : Q][6];
       D3 dv2[kDv ? 1 : Q];
@@ -824,7 +802,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         if (!kNah) vorkond_g(q, p2[kNah ? 0 : q]);
         if (!kDv) dv2[kDv ? 0 : q] = dv_lesen(q);
       }
-      if (!(gut = sammeln<1>(a, sh, ca, seq, SC))) break;
+      if (!(gut = sammeln<1>(a, sh, ca, seq))) break;
       if (ca[0] <= DBL_MIN || !isfinite(ca[0])) {
         brk = true;
         break;
@@ -846,24 +824,6 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         }
         D3 s = ap_lesen(q);
         const D3 n = normale(q);
-        if (SC && (fl[q] & kFrei)) {  // the point's spring entries, in list order
-          const R4<double>* out = static_cast<const R4<double>*>(a.sc_out);
-          D3 f = d3(0.0, 0.0, 0.0);
-          const uint32_t e1 = a.sc_off[pt[q] + 1];
-          uint32_t e = a.sc_off[pt[q]];
-          for (; e + 4 <= e1; e += 4) {
-            R4<double> t[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = out[e + k];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) f = f + d3(t[k].x, t[k].y, t[k].z);
-          }
-          for (; e < e1; ++e) {
-            const R4<double> t = out[e];
-            f = f + d3(t.x, t.y, t.z);
-          }
-          s = s + s_filter(n, f);
-        }
         const D3 rn = d3(r[q][0] - alpha * s.x, r[q][1] - alpha * s.y, r[q][2] - alpha * s.z);
         r[q][0] = rn.x;
         r[q][1] = rn.y;
@@ -924,13 +884,13 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     // held point that pulls on the body is released
     if (!(gut = dv_auslegen())) break;
     produkt<R, Q>(a, sh, g, strom, fest, o);
+    if (SC) federn(ep, 0.0, true);
     double los[1] = {0.0};
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       if (!(fl[q] & kZeile) || !(fl[q] & kGehalten)) continue;
       const D3 n = normale(q);
       D3 ad = d3(o[q][0], o[q][1], o[q][2]);
-      if (SC) ad = ad + federn_dv<R>(a, pt[q]);
       const D3 rest = ad - ld3(a.b, pt[q]);
       const double fn = dot(rest, n) / a.h;
       if (fn < 0.0) {
@@ -980,20 +940,17 @@ const void* fn_of(int rsize, bool sc, int q) {
 
 size_t kachel_kopf_bytes() { return kachel_kopf(sizeof(KSh)); }
 
-size_t kachel_smem(int rsize, int device) {
+size_t kachel_smem(int device) {
   int most = 0;
   if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return 0;
-  for (int sc = 0; sc < 2; ++sc)
-    for (int q = 1; q <= kKachelZeilen; ++q) {
-      const void* fn = fn_of(rsize, sc != 0, q);
-      cudaFuncAttributes at;
-      if (cudaFuncGetAttributes(&at, fn) != cudaSuccess || at.maxThreadsPerBlock < kNT) return 0;
-      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(at.sharedSizeBytes)) !=
-          cudaSuccess)
-        return 0;
-      if (at.sharedSizeBytes != 0) return 0;  // the layout above is all of it
-    }
   return size_t(most);
+}
+
+bool kachel_bereit(int rsize, bool federn, int q, size_t smem) {
+  const void* fn = fn_of(rsize, federn, q);
+  cudaFuncAttributes at;
+  return cudaFuncGetAttributes(&at, fn) == cudaSuccess && at.maxThreadsPerBlock >= kNT && at.sharedSizeBytes == 0 &&
+         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) == cudaSuccess;
 }
 
 cudaError_t launch_kachel(const StepArgs& a, cudaStream_t st) {

@@ -39,8 +39,7 @@ namespace {
 // 16 and 8 MB: 160 k points, FP32 blocks (65 MB streamed) 49.6, 49.3, 47.9,
 // 42.1, 42.9, 45.0; 160 k, FP64 (146 MB) 94.8, -, 77.9, 74.0, 72.5, 72.0;
 // 205 k of a garment, FP32 blocks -, 62.2, 54.7, 52.1, 52.2, 52.5; 90 k, FP64
-// (81 MB) 48.2, -, 43.4, 43.3, 44.0, 41.3; up to 55 MB no difference. So little:
-// each half of the L2 keeps its own copy of what its SMs read.
+// (81 MB) 48.2, -, 43.4, 43.3, 44.0, 41.3; up to 55 MB no difference.
 constexpr size_t kKachelL2 = size_t(24) << 20;
 
 // Splits the points idx[lo, hi) into nb parts of whole slices (the last one
@@ -114,10 +113,9 @@ bool kachelplan(const Spalten& S, const double* x, const std::vector<int64_t>& i
     if (m == 0 || nb < 1) return false;
     for (size_t i = lo; i < hi; ++i) idx[i] = uint32_t(i);
     bool einzeln = false;
-    if (ng > 1 || m <= kKachelNatur) {
-      const bool klein = m <= 512 * nb && ns <= 512 && ns <= nb * warps;
-      einzeln = klein && !federn;
-      if (klein) {
+    if (ng > 1 || (m <= kKachelNatur && !federn)) {
+      einzeln = m <= 512 * nb && ns <= 512 && ns <= nb * warps;
+      if (einzeln) {
         for (size_t s = 0; s < ns; s += warps)
           kachel(&idx[lo + 32 * s], std::min<size_t>(32 * warps, m - 32 * s));
       } else {
@@ -131,7 +129,7 @@ bool kachelplan(const Spalten& S, const double* x, const std::vector<int64_t>& i
       }
     } else {
       std::vector<size_t> anf(1, lo);
-      teile(idx, lo, hi, int(std::min(nb, ns)), x, anf);
+      teile(idx, lo, hi, int(std::min(nb, federn ? (ns + 1) / 2 : ns)), x, anf);
       for (size_t b = 0; b + 1 < anf.size(); ++b) {  // within a tile the points keep their natural order
         std::sort(idx.begin() + std::ptrdiff_t(anf[b]), idx.begin() + std::ptrdiff_t(anf[b + 1]));
         kachel(&idx[anf[b]], anf[b + 1] - anf[b]);
@@ -180,7 +178,7 @@ bool kachelplan(const Spalten& S, const double* x, const std::vector<int64_t>& i
     const size_t ns = (size_t(B.rows) + 31) / 32, s0 = B.row0 / 32, nw = std::min<size_t>(ns, 16);
     const size_t ts = 32 * ns + B.halos;
     if (ts > 65535) return false;
-    const size_t vorn = kopf + kachel_tile(ns, B.halos, kachel_ap(rsize, P.q));
+    const size_t vorn = kopf + kachel_tile(rsize, ns, B.halos, kachel_ap(rsize, P.q), federn);
     if (vorn >= smem) return false;
     const size_t platz = (smem - vorn) / (nw * satz);
     std::vector<uint32_t> breit(ns, 0);

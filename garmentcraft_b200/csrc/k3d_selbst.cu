@@ -1184,6 +1184,119 @@ __global__ void __launch_bounds__(kT) inc_pos_kernel(const __grid_constant__ Sel
   SC_FOR(e, E) s.inc_pos[s.inc_ent[e]] = uint32_t(e);
 }
 
+// ------------------------------------------------------------ springs as rows
+// Each point's entries (spring, slot) merged into one row of 3x3 blocks, the
+// form in which the tiled PCG applies them: a slot of weight g_k couples its
+// point with the spring's points of the other sign (implizit.rs:214-220),
+//   f_k = sum_r om B (c_k - c_r),  om = -g_k g_r,
+// so the row is its diagonal, sum om B, and -om B per neighbour. Springs share
+// their points: 205 k points with 9,335 point-triangle, 27,660 edge-edge and
+// 26,128 push springs have 590,872 couplings of 93,142 pairs of points, at most
+// 14 a row. A warp a row: its lanes load 32 entries at a time, which then pass
+// in list order, and each lane keeps one neighbour; further neighbours take
+// another sweep. Sums in FP64 in list order, so the same bits on every run.
+__global__ void __launch_bounds__(kT) sf_marke_kernel(const __grid_constant__ SelbstArgs s) {
+  SC_FOR(i, s.n + 1) s.sf_nr[i] = i < s.n && s.inc_off[i] != s.inc_off[i + 1] ? 1u : 0u;
+}
+template <typename R>
+__global__ void __launch_bounds__(kT) sf_zeilen_kernel(const __grid_constant__ SelbstArgs s) {
+  const int64_t i = (int64_t(blockIdx.x) * kT + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= s.n) return;
+  const uint32_t e0 = s.inc_off[i], e1 = min(s.inc_off[i + 1], s.cap_inc);
+  if (e0 >= e1) return;
+  const uint32_t zeile = s.sf_nr[i];
+  const size_t anf = 4 * size_t(e0) + zeile;  // at most four neighbours an entry, and the diagonals of the rows before
+  const size_t cap = s.cap_sf;
+  const R4<R>* bR = static_cast<const R4<R>*>(s.pr_bR);
+  const R4<R>* wR = static_cast<const R4<R>*>(s.pr_wR);
+  const R* g5R = static_cast<const R*>(s.pr_g5R);
+  double diag[6] = {};
+  uint32_t fertig = 0;  // neighbours of the sweeps before
+  for (bool rest = true; rest;) {
+    rest = false;
+    uint32_t zahl = 0, mein = 0;
+    double acc[6] = {};
+    for (uint32_t c = e0; c < e1; c += 32) {
+      uint32_t j[4] = {0, 0, 0, 0};
+      double om[4] = {0, 0, 0, 0}, b[6] = {};
+      if (c + lane < e1) {
+        const uint32_t ent = s.inc_ent[c + lane], q = ent >> 3, k = ent & 7u;
+        const uint4 id = s.pr_idx[q];
+        const R4<R> w4 = wR[q], b0 = bR[2 * size_t(q)], b1 = bR[2 * size_t(q) + 1];
+        const double g[5] = {double(w4.x), double(w4.y), double(w4.z), double(w4.w), double(g5R[q])};
+        const uint32_t ix[5] = {id.x, id.y, id.z, id.w, s.pr_x5[q]};
+        const double gk = k == 0 ? g[0] : k == 1 ? g[1] : k == 2 ? g[2] : k == 3 ? g[3] : g[4];
+        b[0] = double(b0.x);
+        b[1] = double(b0.y);
+        b[2] = double(b0.z);
+        b[3] = double(b0.w);
+        b[4] = double(b1.x);
+        b[5] = double(b1.y);
+        int m = 0;
+#pragma unroll
+        for (int r = 0; r < 5; ++r)
+          if ((gk > 0.0 && g[r] < 0.0) || (gk < 0.0 && g[r] > 0.0)) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+              if (t == m) {
+                j[t] = ix[r];
+                om[t] = -gk * g[r];
+              }
+            ++m;
+          }
+      }
+      const uint32_t mt = min(32u, e1 - c);
+      for (uint32_t t = 0; t < mt; ++t) {
+        double bt[6];
+#pragma unroll
+        for (int x = 0; x < 6; ++x) bt[x] = __shfl_sync(0xffffffffu, b[x], int(t));
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const double o = __shfl_sync(0xffffffffu, om[m], int(t));
+          const uint32_t jj = __shfl_sync(0xffffffffu, j[m], int(t));
+          if (o == 0.0) continue;
+          if (fertig == 0)
+#pragma unroll
+            for (int x = 0; x < 6; ++x) diag[x] += o * bt[x];
+          unsigned wer = __ballot_sync(0xffffffffu, uint32_t(lane) < zahl && mein == jj);
+          if (wer == 0) {
+            bool da = false;
+            for (uint32_t p = 0; p < fertig && !da; p += 32)
+              da = __any_sync(0xffffffffu, p + lane < fertig && s.sf_spalte[anf + 1 + p + lane] == jj);
+            if (da) continue;
+            if (zahl == 32) {
+              rest = true;
+              continue;
+            }
+            if (uint32_t(lane) == zahl) mein = jj;
+            wer = 1u << zahl;
+            ++zahl;
+          }
+          if ((wer >> lane) & 1u)
+#pragma unroll
+            for (int x = 0; x < 6; ++x) acc[x] += o * bt[x];
+        }
+      }
+    }
+    if (uint32_t(lane) < zahl) {
+      const size_t p = anf + 1 + fertig + lane;
+      s.sf_spalte[p] = mein;
+#pragma unroll
+      for (int x = 0; x < 6; ++x) s.sf_block[x * cap + p] = -acc[x];
+    }
+    fertig += zahl;
+    __syncwarp();
+  }
+  if (lane == 0) {
+    s.sf_spalte[anf] = uint32_t(i);
+#pragma unroll
+    for (int x = 0; x < 6; ++x) s.sf_block[x * cap + anf] = diag[x];
+    s.sf_anf[zeile] = uint32_t(anf);
+    s.sf_anz[zeile] = 1 + fertig;
+  }
+}
+
 // ------------------------------------------------------------ exclusive scan
 // Exclusive prefix sum of n uint32 in place, 1024 per block; block totals in
 // tmp, scanned by one block; `total` receives the sum.
@@ -2322,7 +2435,9 @@ cudaError_t exclusive_scan_u32(uint32_t* data, int64_t n, uint32_t* tmp, uint32_
 // count, scan, fill, sort
 // (+3 and +2: the entry boxes of the point, edge and triangle hashes and of
 // the two path hashes)
-int selbst_launches_per_run() { return 2 + (6 + 3 + 6 + 10) + (4 + 12 + 3 + 3) + 6 + 4 + 3; }
+int selbst_launches_per_run(bool zeilen) {
+  return 2 + (6 + 3 + 6 + 10) + (4 + 12 + 3 + 3) + 6 + 4 + 3 + (zeilen ? 4 : 0);
+}
 int selbst_stoss_launches(int iterationen) { return 8 + 6 + 4 + 3 + 3 + 3 * iterationen + 1 + 3 + 2 + 2; }
 
 // Impacts, part 1 (selbstkollision.rs:1196-1203): the longest edge at x1, the
@@ -2477,7 +2592,18 @@ cudaError_t selbst_paare_und_federn(const SelbstArgs& s, uint32_t n_aktiv_p, uin
   inc_fill_kernel<<<grid_for(pmax), kT, 0, st>>>(s);
   inc_sort_kernel<<<grid_for(s.n), kT, 0, st>>>(s);
   if ((e = lang_sort(s.inc_off, s.inc_ent, s.n, st)) != cudaSuccess) return e;
-  inc_pos_kernel<<<grid_for(int64_t(s.cap_inc)), kT, 0, st>>>(s);
+  if (!s.zeilen) {
+    inc_pos_kernel<<<grid_for(int64_t(s.cap_inc)), kT, 0, st>>>(s);
+    return cudaGetLastError();
+  }
+  sf_marke_kernel<<<grid_for(s.n + 1), kT, 0, st>>>(s);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = scan(s.sf_nr, s.n + 1, s.scan_tmp, nullptr, st)) != cudaSuccess) return e;
+  const unsigned blk = unsigned((s.n + kT / 32 - 1) / (kT / 32));
+  if (s.rsize == 4)
+    sf_zeilen_kernel<float><<<blk, kT, 0, st>>>(s);
+  else
+    sf_zeilen_kernel<double><<<blk, kT, 0, st>>>(s);
   return cudaGetLastError();
 }
 

@@ -106,7 +106,13 @@ struct SelbstArgs {
   uint32_t cap_inc;
   uint32_t* inc_pos;  // per (spring << 3 | slot): its entry index, all ones for a zero weight
   void* inc_out;      // per entry: the PCG's spring product of that slot, R4
-  double* pr_c;       // the PCG direction at each spring's five points: 15 planes of cap_pairs
+  // the springs as rows of merged blocks, for the tiled PCG (zeilen != 0): row
+  // k of the points with entries has sf_anz[k] blocks from sf_anf[k] on, the
+  // diagonal first; sf_nr: per point its row, then the rows' count (n + 1)
+  int zeilen;
+  uint32_t cap_sf;
+  uint32_t *sf_nr, *sf_anf, *sf_anz, *sf_spalte;
+  double* sf_block;  // symmetric blocks (xx, yy, zz, xy, xz, yz): 6 planes of cap_sf
   int32_t* slot_of;  // damping scratch per point: its shared-memory slot, -1 between batches
   uint32_t* zahl;    // SZ_COUNT counters
   uint32_t* scan_tmp;
@@ -161,7 +167,7 @@ cudaError_t selbst_hash_fuellen_und_paare_zaehlen(const SelbstArgs& s, cudaStrea
 // n_s: the intersections (counter SZ_SCHNITTE, at most cap_s)
 cudaError_t selbst_paare_und_federn(const SelbstArgs& s, uint32_t n_aktiv_p, uint32_t n_aktiv_s, uint32_t n_s,
                                     cudaStream_t st);
-int selbst_launches_per_run();
+int selbst_launches_per_run(bool zeilen);
 // Impacts after the step's integration, in two parts with a host read of the
 // path hashes' entry counts between them.
 cudaError_t selbst_stoss_zaehlen(const SelbstArgs& s, cudaStream_t st);

@@ -46,6 +46,7 @@ void selbst_free(SelbstHost& H) {
   free_all(H.fest);
   free_all(H.pairs);
   free_all(H.hashk);
+  free_all(H.sf);
   free_all(H.schn);
   free_all(H.wege);
   H.on = false;
@@ -422,8 +423,22 @@ cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap) {
   char* out = nullptr;
   if ((e = alloc(out, size_t(s.cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
   s.inc_out = out;
-  if ((e = alloc(s.pr_c, size_t(15) * cap, H.pairs)) != cudaSuccess) return e;
   return alloc(s.inc_ent, size_t(s.cap_inc), H.pairs);
+}
+
+cudaError_t selbst_grow_zeilen(SelbstHost& H, uint32_t cap) {
+  free_all(H.sf);
+  SelbstArgs& s = H.s;
+  const size_t n = size_t(s.n);
+  cudaError_t e;
+  if ((e = alloc(s.sf_nr, n + 1, H.sf)) != cudaSuccess) return e;
+  if ((e = alloc(s.sf_anf, n, H.sf)) != cudaSuccess) return e;
+  if ((e = alloc(s.sf_anz, n, H.sf)) != cudaSuccess) return e;
+  if ((e = alloc(s.sf_spalte, size_t(cap), H.sf)) != cudaSuccess) return e;
+  if ((e = alloc(s.sf_block, size_t(cap) * 6, H.sf)) != cudaSuccess) return e;
+  s.cap_sf = cap;
+  s.zeilen = 1;
+  return cudaSuccess;
 }
 
 cudaError_t selbst_set_naht_ruhe(SelbstHost& H, const double* ruhe, int64_t n_naht, cudaStream_t st) {
@@ -472,6 +487,14 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
     if (want > 0x1fffffffu) return cudaErrorMemoryAllocation;
     if ((e = selbst_grow_pairs(H, uint32_t(want))) != cudaSuccess) return e;
   }
+  if (s.zeilen) {  // at most four blocks for each nonzero slot, and a diagonal for each point
+    const uint64_t most = 4 * (4 * paare + 5 * uint64_t(n_s)) + uint64_t(s.n);
+    if (most > s.cap_sf) {
+      const uint64_t want = most + most / 2;
+      if (want > 0xffffffffu) return cudaErrorMemoryAllocation;
+      if ((e = selbst_grow_zeilen(H, uint32_t(want))) != cudaSuccess) return e;
+    }
+  }
   if ((e = cudaMemsetAsync(s.inc_off, 0, sizeof(uint32_t) * (size_t(s.n) + 1), st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(s.inc_cur, 0, sizeof(uint32_t) * size_t(s.n), st)) != cudaSuccess) return e;
   if (federn > 0 && (e = cudaMemsetAsync(s.inc_pos, 0xff, sizeof(uint32_t) * 8 * size_t(federn), st)) != cudaSuccess)
@@ -488,7 +511,7 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
   H.naehe_pt += z[SZ_PAARE_PT];
   H.naehe_kk += z[SZ_PAARE_KK];
   H.ran = true;
-  launches += selbst_launches_per_run();
+  launches += selbst_launches_per_run(s.zeilen != 0);
   return cudaSuccess;
 }
 
@@ -528,8 +551,9 @@ void selbst_step_args(const SelbstHost& H, StepArgs& a) {
     a.sc_w = a.sc_kf = a.sc_b0 = a.sc_b1 = nullptr;
     a.sc_bR = a.sc_wR = nullptr;
     a.sc_out = nullptr;
-    a.sc_c = nullptr;
-    a.sc_cap = 0;
+    a.sf_zahl = a.sf_anf = a.sf_anz = a.sf_spalte = nullptr;
+    a.sf_block = nullptr;
+    a.sf_cap = 0;
     a.sc_np = 0;
     a.sc_x5 = nullptr;
     a.sc_g5 = nullptr;
@@ -548,8 +572,12 @@ void selbst_step_args(const SelbstHost& H, StepArgs& a) {
   a.sc_wR = s.pr_wR;
   a.sc_pos = s.inc_pos;
   a.sc_out = s.inc_out;
-  a.sc_c = s.pr_c;
-  a.sc_cap = s.cap_pairs;
+  a.sf_zahl = s.zeilen ? s.sf_nr + s.n : nullptr;
+  a.sf_anf = s.sf_anf;
+  a.sf_anz = s.sf_anz;
+  a.sf_spalte = s.sf_spalte;
+  a.sf_block = s.sf_block;
+  a.sf_cap = s.cap_sf;
   a.sc_x5 = s.pr_x5;
   a.sc_g5 = s.pr_g5;
   a.sc_g5R = s.pr_g5R;

@@ -13,7 +13,7 @@ struct SelbstHost {
   bool on = false;   // tables uploaded (ImplizitParameter::selbstkollision)
   bool ran = false;  // a run has filled the pair buffers
   SelbstArgs s{};
-  std::vector<void*> fest, pairs, hashk;  // device allocations: fixed, pair-sized, edge-hash
+  std::vector<void*> fest, pairs, hashk, sf;  // device allocations: fixed, pair-sized, edge-hash, merged rows
   std::vector<void*> schn, wege;          // intersection-sized; path-hash entries
   double* x0 = nullptr;                   // positions at the start of the substep
   Body* bodies_dev = nullptr;             // the substep's bodies (pinch test)
@@ -34,6 +34,8 @@ cudaError_t selbst_grow_edge_hash(SelbstHost& H, uint32_t cap);
 cudaError_t selbst_grow_schnitte(SelbstHost& H, uint32_t cap);
 cudaError_t selbst_grow_wege(SelbstHost& H, uint32_t cap_p, uint32_t cap_k);
 cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap);
+// Room for the springs as rows of merged blocks (the tiled PCG applies these).
+cudaError_t selbst_grow_zeilen(SelbstHost& H, uint32_t cap);
 cudaError_t selbst_set_naht_ruhe(SelbstHost& H, const double* ruhe, int64_t n_naht, cudaStream_t st);
 // One run on the current state with substep h (two host reads of the counts).
 cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches);

@@ -74,9 +74,16 @@ __host__ __device__ constexpr unsigned kachel_satz(size_t rsize) { return unsign
 __host__ __device__ constexpr size_t kachel_kopf(size_t bytes) { return (bytes + 127) & ~size_t(127); }
 // A c beside the tile in shared memory, where the registers are short
 __host__ __device__ constexpr bool kachel_ap(size_t rsize, int q) { return q > 2 || (rsize == 8 && q > 1); }
-// the tile's bytes: ns slices and halos, and A c of the slices
-__host__ __device__ constexpr size_t kachel_tile(size_t ns, size_t halos, bool ap) {
-  return (24 * (32 * ns * (ap ? 2 : 1) + halos) + 127) & ~size_t(127);
+// With self-collision a CTA keeps the heads of its first rows of merged spring
+// blocks (start, blocks, the first columns).
+constexpr int kFederZeilen = 96, kFederSpalten = 8;
+// the tile's bytes: ns slices and halos, A c of the slices, the springs' part of
+// it (FP64 blocks), and the heads of the springs' rows, in this order
+__host__ __device__ constexpr size_t kachel_vektoren(size_t rsize, size_t ns, size_t halos, bool ap, bool federn) {
+  return (24 * (32 * ns * size_t(1 + ap + (federn && rsize == 8)) + halos) + 127) & ~size_t(127);
+}
+__host__ __device__ constexpr size_t kachel_tile(size_t rsize, size_t ns, size_t halos, bool ap, bool federn) {
+  return kachel_vektoren(rsize, ns, halos, ap, federn) + (federn ? size_t(kFederZeilen) * (8 + 4 * kFederSpalten) : 0);
 }
 struct KachelBlk {
   uint32_t row0, rows;    // first position (a multiple of 32) and rows of the tile
@@ -202,12 +209,16 @@ struct StepArgs {
   // one after another, and so do its resident ones
   const uint4* ka_slice;
   const uint16_t* ka_lc;
-  ulonglong2* ka_wort;      // published vectors: 2 x 3 planes of n words
+  ulonglong2* ka_wort;      // published vectors: 2 x 3 planes of n words (with self-collision twice that)
   ulonglong2* ka_summe;     // posted partial sums: 2 x 2 x kKachelKopien x kKachelWorte
   void* ka_pv;              // the preconditioner in position order: 6 planes of 32 ka_slices
   double* ka_dv;            // dv likewise: 3 planes
-  double* sc_c;             // c of each spring's five points: 15 planes of sc_cap
-  int64_t sc_cap, ka_slices;
+  int64_t ka_slices;
+  // the self-collision springs as rows of merged blocks (SelbstArgs::sf_*);
+  // their products are published after ka_wort's vectors, in as many planes
+  const uint32_t *sf_zahl, *sf_anf, *sf_anz, *sf_spalte;
+  const double* sf_block;
+  int64_t sf_cap;
   int ka_blocks, ka_q, ka_smem, ka_rsize;
   // bookkeeping
   cudaEvent_t ev_solve0, ev_solve1;  // around the PCG launch (host-side handles)
@@ -229,9 +240,11 @@ int step_grid_blocks(int precision, int threads, int device);
 // Enqueues one substep (or probe) on `stream`; `launched` = kernels enqueued.
 cudaError_t launch_step(const StepArgs& a, int precision, int blocks, cudaStream_t stream, int& launched);
 // The tiled PCG: its shared header's size, the dynamic shared memory a CTA
-// can take (0: not available here), and its launch.
+// can take (0: not available here), whether its kernel can take it (and is set
+// to; the other forms' kernels are not loaded), and its launch.
 size_t kachel_kopf_bytes();
-size_t kachel_smem(int rsize, int device);
+size_t kachel_smem(int device);
+bool kachel_bereit(int rsize, bool federn, int q, size_t smem);
 cudaError_t launch_kachel(const StepArgs& a, cudaStream_t stream);
 // The FP64 PCG launch alone on the system built before (one pass, no release
 // test): dv (start and result), b, normals and the assembled A as in `a`.

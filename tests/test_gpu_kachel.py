@@ -104,3 +104,19 @@ def test_stapel(prec):
         gleich(a[0], b[0], "dv")
         gleich(a[2], b[2], "x")
 
+
+
+# (side, edge, extra thickness, CTAs): layers in light contact; a few points;
+# springs to more than 32 neighbours a point; one and three CTAs, with more rows
+# of springs than a CTA keeps the heads of, on one and three rows a thread
+@pytest.mark.parametrize("groesse, kante_mm, dicke, bloecke", [
+    (0.2, 10.0, 4e-3, 0), (0.02, 10.0, 4e-3, 0), (0.1, 5.0, 2.5e-2, 0), (0.15, 10.0, 1e-2, 1), (0.2, 5.0, 6e-3, 3)])
+@pytest.mark.parametrize("prec", FORMEN)
+def test_selbstkollision(prec, groesse, kante_mm, dicke, bloecke):
+    s = build_scene(synth.zwei_lagen(groesse_m=groesse, kante_mm=kante_mm, abstand_m=0.003, versatz_m=(0.0013, 0.0007)))
+    synth.pin_teil(s, 0)
+    s.v[:] = np.random.default_rng(2).normal(0.0, 0.02, size=s.v.shape)
+    s.param.bild_dt = 1.0 / 600.0
+    a, b = beide(s, prec, selbstkollision=True, selbst_zusatzdicke=dicke, pcg_bloecke=bloecke)
+    assert a[1] == b[1]
+    gleich(a[0], b[0], "dv")
