@@ -232,7 +232,7 @@ def garment_leg(flush, torch, peaks, cpu=True):
                         "pcg_ms_per_step": sms / GARMENT_STEPS}
             if selbst and prec == HEADLINE:
                 out["roofline"] = roofline_of(s, prec, its, solves, sms, sum(ms), GARMENT_STEPS, peaks,
-                                              "k3d::solve_kernel<float, double, true>")
+                                              "k3d::kachel_kernel<float, true, Q>")
             del cg
     for tag in ("selfcollision", "no_selfcollision"):
         for prec in (HEADLINE, 1):
@@ -990,7 +990,7 @@ def main():
 
     peaks = read_peaks()
     roofline = roofline_of(s_h, HEADLINE, its, solves, cg.solve_ms_total, sum(ms), a.steps, peaks,
-                           "k3d::solve_kernel<float, double, false>")
+                           "k3d::kachel_kernel<float, false, Q>")
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": 1e3 * t_dev / a.steps, "higher_is_better": True,
