@@ -70,13 +70,20 @@ __global__ void __launch_bounds__(kT) flaechen_kernel(const __grid_constant__ De
     }
     const D3 A = kl == 0 ? q[0] : kl == 1 ? q[1] : q[2], B = kl == 0 ? q[1] : kl == 1 ? q[2] : q[0],
              C = kl == 0 ? q[2] : kl == 1 ? q[0] : q[1];
-    const D3 ua = normiert(B - A), va = cross(n, ua);
+    // On corners that are collinear up to rounding the cross product is rounding
+    // noise, and n as it stands has any part along u (the bound then counts
+    // distance along the edge and rules out the nearest triangle). Its part along
+    // u is taken out twice, as the first time may leave no more than noise again.
+    const D3 ua = normiert(B - A);
+    D3 na = normiert(n - ua * dot(n, ua));
+    na = normiert(na - ua * dot(na, ua));
+    const D3 va = cross(na, ua);
     const double cu = dot(C - A, ua), cv = dot(C - A, va);
     const double lb = hypot(cv, ll - cu), lc = hypot(cv, cu);
     const double b0 = lb > 0.0 ? cv / lb : 0.0, b1 = lb > 0.0 ? (ll - cu) / lb : 0.0;
     const double c0 = lc > 0.0 ? -cv / lc : 0.0, c1 = lc > 0.0 ? cu / lc : 0.0;
     float4* ef = g.ef + kEben * t;
-    ef[0] = make_float4(float(n.x), float(n.y), float(n.z), float(-dot(n, A)));
+    ef[0] = make_float4(float(na.x), float(na.y), float(na.z), float(-dot(na, A)));
     ef[1] = make_float4(float(ua.x), float(ua.y), float(ua.z), float(-dot(ua, A)));
     ef[2] = make_float4(float(va.x), float(va.y), float(va.z), float(-dot(va, A)));
     ef[3] = make_float4(float(ll), float(cv), float(b0), float(b1));
@@ -281,8 +288,9 @@ __device__ __forceinline__ void schreibe(const Treffer& r, int64_t q, double* ab
 // A lower bound of the distance from x to a triangle in FP32: its distance to
 // the plane and, within the plane, to the rectangle on the longest edge or
 // outside one of the other edges, whichever is more (exact but for small parts
-// of the corners' regions, on slivers too). `weg` covers the rounding of x, of
-// the frame and of the products: 16 ulp of the largest coordinate that occurs.
+// of the corners' regions, on slivers too; on corners collinear up to rounding
+// it is the distance to the segment). `weg` covers the rounding of x, of the
+// frame and of the products: 16 ulp of the largest coordinate that occurs.
 struct Naehe {
   float x, y, z, weg;
   __device__ Naehe(const Dev& g, D3 p) : x(float(p.x)), y(float(p.y)), z(float(p.z)) {
