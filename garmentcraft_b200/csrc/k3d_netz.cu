@@ -290,11 +290,14 @@ __device__ __forceinline__ void schreibe(const Treffer& r, int64_t q, double* ab
 // outside one of the other edges, whichever is more (exact but for small parts
 // of the corners' regions, on slivers too; on corners collinear up to rounding
 // it is the distance to the segment). `weg` covers the rounding of x, of the
-// frame and of the products: 16 ulp of the largest coordinate that occurs.
+// frame and of the products: 16 ulp of the largest coordinate that occurs. Where
+// its square or that rounding leaves FP32's range the bound is 0, and the FP64
+// test decides alone.
 struct Naehe {
   float x, y, z, weg;
   __device__ Naehe(const Dev& g, D3 p) : x(float(p.x)), y(float(p.y)), z(float(p.z)) {
-    weg = 2e-6f * fmaxf(g.weit, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))));
+    const float m = fmaxf(g.weit, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))));
+    weg = m > 1e-18f && m < 1e18f ? 2e-6f * m : INFINITY;
   }
   __device__ float abstand(const float4* e) const {
     auto s = [&](float4 k) { return __fmaf_rn(k.x, x, __fmaf_rn(k.y, y, __fmaf_rn(k.z, z, k.w))); };

@@ -88,3 +88,29 @@ def test_sdf(netz):
         nah = np.abs(exakt) < 0.02  # beyond the band an open surface has no side
         assert nah.sum() > 500
         assert np.array_equal(a[nah], b[nah]) and np.array_equal(np.abs(a), np.abs(b))
+
+
+# Sizes whose coordinates, squares or roundings leave the range of 32 bits
+@pytest.mark.parametrize("masstab", [1e-42, 1e-25, 1e25, 1e40])
+def test_masstab(masstab):
+    p, d = synth.koerper_netz(48, 17, seed=6)
+    x = anfragen(p, d, np.arange(len(d)), 3000, np.random.default_rng(2))
+    kg, ko = Koerpernetz(p * masstab, d, 0.01 * masstab), O.Koerpernetz(p * masstab, d, 0.01 * masstab)
+    a, b = kg.naechster(x * masstab, 0.008 * masstab), ko.naechster(x * masstab, 0.008 * masstab)
+    assert 0.5 < (b["dreieck"] >= 0).mean() < 1.0
+    for k in WERTE:
+        assert np.array_equal(a[k], b[k]), k
+    o, s, band = p[0] * masstab, 0.004 * masstab, 0.02 * masstab
+    assert np.array_equal(kg.sdf((9, 8, 7), o, s, band=band), ko.sdf((9, 8, 7), o, s, band=band))
+
+
+@pytest.mark.parametrize("weit", [1e10, 1e22])
+def test_ferne_anfragen(weit):
+    p, d = synth.koerper_netz(24, 9, seed=6)
+    kg, ko = Koerpernetz(p, d, 0.01), O.Koerpernetz(p, d, 0.01)
+    x = np.random.default_rng(3).normal(size=(50, 3))
+    x *= weit / np.linalg.norm(x, axis=1)[:, None]
+    a, b = kg.naechster(x, 2.0 * weit), ko.naechster(x, 2.0 * weit)
+    assert (b["dreieck"] >= 0).all()
+    for k in WERTE:
+        assert np.array_equal(a[k], b[k]), k
