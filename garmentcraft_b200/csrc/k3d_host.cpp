@@ -966,11 +966,15 @@ static k3d_status check_sync(k3d_solver* h) {
   SyncState ss;
   K3D_CUDA(h, cudaMemcpy(&ss, h->a.sync, sizeof(ss), cudaMemcpyDeviceToHost));
   if (ss.error != 0) {
-    cudaMemset(&h->a.sync->error, 0, sizeof(int));
+    // on the handle's own stream, which the next launch follows (it does not
+    // wait for the legacy stream)
+    K3D_CUDA(h, cudaMemsetAsync(&h->a.sync->error, 0, sizeof(int), h->stream));
     if (h->a.ka_blk) {  // the sequence numbers of a launch that gave up start again
-      cudaMemset(h->a.ka_wort, 0, sizeof(ulonglong2) * (h->p.selbstkollision ? 12 : 6) * size_t(h->n));
-      cudaMemset(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte));
-      cudaMemset(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp));
+      K3D_CUDA(h, cudaMemsetAsync(h->a.ka_wort, 0, sizeof(ulonglong2) * (h->p.selbstkollision ? 12 : 6) * size_t(h->n),
+                                  h->stream));
+      K3D_CUDA(h, cudaMemsetAsync(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte),
+                                  h->stream));
+      K3D_CUDA(h, cudaMemsetAsync(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp), h->stream));
     }
     return fail(h, K3D_TIMEOUT, "a device barrier wait ran out of time");
   }
