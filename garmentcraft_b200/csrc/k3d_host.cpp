@@ -46,6 +46,8 @@ struct k3d_solver {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err, name;
   int blocks = 0;
+  uint64_t frist_ns = kBarrierLimitNs;  // StepArgs
+  int64_t stumm_nach = -1;
   size_t ka_smem = 0;  // shared memory a CTA of the tiled PCG takes (0: the launch over ELL rows)
   size_t rsize = 8;  // operator records, assembled blocks, preconditioner
   size_t vsize = 8;  // the PCG's vectors
@@ -900,6 +902,8 @@ static void step_args(k3d_solver* h, int mode, double t_bodies, bool need_load) 
   a.durchstoss_pruefen = h->p.durchstoss_pruefen ? 1 : 0;
   a.kp_passes = a.kp_nt > 0 ? std::max(h->p.koerperpunkt_durchgaenge, 0) : 0;
   a.kp_tief = h->p.koerperpunkt_tiefe;
+  a.frist_ns = h->frist_ns;
+  a.stumm_nach = h->stumm_nach;
   for (int b = 0; b < a.n_bodies; ++b) {
     const k3d_body& k = h->bodies[b];
     Body& d = a.bodies[b];
@@ -1635,6 +1639,14 @@ k3d_status k3d_adjoint_backward(k3d_solver* h, const double* gx, const double* g
     out->ms_neuberechnung = ms_re;
   }
   return K3D_OK;
+}
+
+// For the library's tests, not part of the ABI that the headers declare: the
+// tiled PCG's waits last `sekunden` at most, and after iteration `nach` (-1: never)
+// one of a solve's sums waits for a word that nobody posts.
+void k3d_test_wait(k3d_solver* h, double sekunden, int64_t nach) {
+  h->frist_ns = uint64_t(sekunden * 1e9);
+  h->stumm_nach = nach;
 }
 
 }  // extern "C"

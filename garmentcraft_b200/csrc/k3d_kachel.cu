@@ -36,8 +36,12 @@
 // point, 205 k points with 63 k springs, 3051 iterations, took 217 ms, here
 // 117 ms; two layers of 3 k points, 907 iterations in ten solves, 30 ms and 16.
 // Sums are deterministic: a fixed tree per CTA, then the CTAs' partials in
-// CTA order in every CTA. Every wait is bounded (kBarrierLimitNs): it records
-// K3D_TIMEOUT, the warps wait for their copies in flight, and all return.
+// CTA order in every CTA. Every wait is bounded (StepArgs::frist_ns). One that
+// gives up records K3D_TIMEOUT, and the others, which look at that record now and
+// then, give up too; waits for a warp's own copies do not, so no CTA leaves with
+// copies under way into its shared memory. The CTA's threads leave together: a
+// barrier lies between each look at sh.err and the next wait that may set it. A
+// launch that finds the record set returns before its first copy.
 #include "k3d_solve.cuh"
 
 namespace k3d {
@@ -82,7 +86,7 @@ __device__ __forceinline__ bool ld_wort(const ulonglong2* p, uint32_t ep, double
   return uint32_t(x >> 32) == ep && uint32_t(y >> 32) == ep;
 }
 
-// A bounded wait: false when it is to give up (another wait did, or time is out).
+// A bounded wait for another CTA: false when it is to give up (another wait did, or time is out).
 struct Warten {
   unsigned n = 0;
   uint64_t t0 = 0;
@@ -93,11 +97,16 @@ __device__ __forceinline__ bool weiter(const StepArgs& a, KSh& sh, Warten& w) {
   const int e = ld_relaxed_i32(&a.sync->error);
   const uint64_t t = globaltimer();
   if (w.t0 == 0) w.t0 = t;
-  if (e == 0 && t - w.t0 <= kBarrierLimitNs) return true;
+  if (e == 0 && t - w.t0 <= a.frist_ns) return true;
   if (e == 0) atomicCAS(&a.sync->error, 0, K3D_STATUS_TIMEOUT);
   *reinterpret_cast<volatile int*>(&sh.err) = K3D_STATUS_TIMEOUT;
   return false;
 }
+// Whether a wait of the CTA gave up. ohne_abbruch is the same in every thread
+// where a barrier lies before it and another before the next wait; einig is both
+// (its vote costs 400 cycles more than a barrier, so the loop has none).
+__device__ __forceinline__ bool ohne_abbruch(KSh& sh) { return *reinterpret_cast<volatile int*>(&sh.err) == 0; }
+__device__ __forceinline__ bool einig(KSh& sh) { return __syncthreads_or(ohne_abbruch(sh) ? 0 : 1) == 0; }
 __device__ __forceinline__ double hol_wort(const StepArgs& a, KSh& sh, const ulonglong2* p, uint32_t ep) {
   double v;
   Warten w;
@@ -156,9 +165,9 @@ __device__ __forceinline__ void melden(const StepArgs& a, KSh& sh, double (&v)[N
   }
 }
 // The sums posted under `seq` by every CTA of the group, the same bits in
-// every thread; false on a timeout. Double-buffered by the number's parity: a
-// CTA posts seq + 2 only after it has waited for seq + 1, which every CTA
-// posts after its wait for seq.
+// every thread (after a wait that gave up too, of no meaning then). Double-buffered
+// by the number's parity: a CTA posts seq + 2 only after it has waited for seq + 1,
+// which every CTA posts after its wait for seq.
 // `vor`: this thread's part of the first sum as it was read ahead (vorab).
 struct Vorab {
   double v = 0.0;
@@ -169,7 +178,7 @@ __device__ __forceinline__ void vorab(const StepArgs& a, const KSh& sh, Vorab& v
     v.da = ld_wort(summe(a, seq, sh.bidx % kKachelKopien, 0) + sh.b.gruppe0 + threadIdx.x, seq, v.v);
 }
 template <int NV>
-__device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq,
+__device__ __forceinline__ void sammeln(const StepArgs& a, KSh& sh, double (&v)[NV], uint32_t seq,
                                         Vorab vor = Vorab()) {
   const unsigned nb = sh.b.worte, lane = threadIdx.x & 31;
   const bool einzeln = sh.b.einzeln != 0;
@@ -181,7 +190,6 @@ __device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[
                                       : hol_wort(a, sh, summe(a, seq, sh.bidx % kKachelKopien, k) + sh.b.gruppe0 + threadIdx.x, seq);
   }
   __syncthreads();
-  if (*reinterpret_cast<volatile int*>(&sh.err) != 0) return false;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     double x = 0.0;
@@ -199,7 +207,6 @@ __device__ __forceinline__ bool sammeln(const StepArgs& a, KSh& sh, double (&v)[
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     v[k] = x;
   }
-  return true;
 }
 
 // ------------------------------------------------------------ the blocks of a warp
@@ -272,9 +279,18 @@ __device__ __forceinline__ void band_start(Band& g, unsigned long long* bar, int
     if (++s == g.stufen) s = 0;
   }
 }
+// A wait for this warp's own copies. They end whatever else has failed, so it
+// gives up only when its own time is out.
 __device__ __forceinline__ void bar_warte(const StepArgs& a, KSh& sh, unsigned long long* b, unsigned par) {
   Warten w;
-  while (!bar_da(b, par) && weiter(a, sh, w)) {
+  while (!bar_da(b, par)) {
+    if ((++w.n & 63u) != 0u) continue;
+    const uint64_t t = globaltimer();
+    if (w.t0 == 0) w.t0 = t;
+    if (t - w.t0 <= a.frist_ns) continue;
+    atomicCAS(&a.sync->error, 0, K3D_STATUS_TIMEOUT);
+    *reinterpret_cast<volatile int*>(&sh.err) = K3D_STATUS_TIMEOUT;
+    return;
   }
 }
 
@@ -426,7 +442,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
   constexpr bool kAp = kachel_ap(sizeof(R), Q);  // A c in shared memory
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    sh.err = 0;
+    sh.err = ld_relaxed_i32(&a.sync->error);
     sh.g = a.grp[a.blk_grp[blockIdx.x]];
     sh.b = a.ka_blk[blockIdx.x];
     sh.bidx = blockIdx.x - sh.g.first_blk;
@@ -440,6 +456,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (!ohne_abbruch(sh)) return;  // a launch before this one gave up
   const unsigned ns = (sh.b.rows + 31) >> 5, halos = sh.b.halos, ts = 32 * ns + halos;
   const uint32_t slice0 = sh.b.row0 >> 5;
   double* tile = reinterpret_cast<double*>(g_roh + kachel_kopf(sizeof(KSh)));
@@ -616,8 +633,7 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     }
     halo_holen();
     if (SC) federzeilen(a, sh, fkopf, ep);
-    __syncthreads();
-    return *reinterpret_cast<volatile int*>(&sh.err) == 0;
+    return einig(sh);
   };
 
   bool gut = true;
@@ -721,10 +737,6 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         halo_holen();
         if (SC) federzeilen(a, sh, fkopf, ep);
         __syncthreads();
-        if (*reinterpret_cast<volatile int*>(&sh.err) != 0) {
-          gut = false;
-          break;
-        }
         vorab(a, sh, vor, seq);  // its latency passes under the product
         produkt<R, Q>(a, sh, g, strom, fest, o);
         if (SC) federn(ep, 0.0, true);
@@ -734,13 +746,13 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
       }
       if (erste) {
         double s[2];
-        if (!(gut = sammeln<2>(a, sh, s, seq, vor))) break;
+        sammeln<2>(a, sh, s, seq, vor);
         delta = s[0];
         bb = s[1];
         ziel = fmax(a.tol * a.tol * fmax(bb, delta), sh.g.boden);
       } else {
         double s[1];
-        if (!(gut = sammeln<1>(a, sh, s, seq, vor))) break;
+        sammeln<1>(a, sh, s, seq, vor);
         beta = s[0] / delta;
         delta = s[0];
         ++it;
@@ -761,10 +773,6 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
           halo[3 * t + 2] = fmar(beta, halo[3 * t + 2], hw.z);
         }
         __syncthreads();
-        if (*reinterpret_cast<volatile int*>(&sh.err) != 0) {
-          gut = false;
-          break;
-        }
         produkt<R, Q>(a, sh, g, strom, fest, o);
         if (SC) federn(ep, beta, false);
       }
@@ -802,7 +810,8 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         if (!kNah) vorkond_g(q, p2[kNah ? 0 : q]);
         if (!kDv) dv2[kDv ? 0 : q] = dv_lesen(q);
       }
-      if (!(gut = sammeln<1>(a, sh, ca, seq))) break;
+      sammeln<1>(a, sh, ca, seq);
+      if (!ohne_abbruch(sh)) break;  // the iteration's waits; melden's barrier lies before the next
       if (ca[0] <= DBL_MIN || !isfinite(ca[0])) {
         brk = true;
         break;
@@ -841,13 +850,14 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
         }
         rz[0] += rn.x * z.x + rn.y * z.y + rn.z * z.z;
       }
+      if (it == a.stumm_nach && threadIdx.x == 0) ++sh.b.worte;
       ++seq;
       melden<1>(a, sh, rz, seq);
       // the next product's first copies travel with the halo and this sum; the
       // update above ran on a quiet memory system
       band_start<R, U>(g, sh.bar[warp], lane);
     }
-    if (!gut) break;
+    if (!(gut = einig(sh))) break;
     // |dv| maximum and the counters go to the statistics by atomics (the
     // groups of a batch finish at different times)
     double dvm = 0.0;
@@ -905,14 +915,15 @@ __global__ void __launch_bounds__(kNT, 1) kachel_kernel(const __grid_constant__ 
     }
     ++seq;
     melden<1>(a, sh, los, seq);
-    if (!(gut = sammeln<1>(a, sh, los, seq))) break;
+    sammeln<1>(a, sh, los, seq);
+    if (!(gut = einig(sh))) break;
     if (lead && los[0] > 0.0)
       atomicAdd(reinterpret_cast<unsigned long long*>(&a.stats[ST_RELEASED]), (unsigned long long)los[0]);
     if (los[0] == 0.0) break;
   }
   // the sequence numbers go on from here in the next launch
   if (lead && gut) *sh.g.count = (ep - ep0 > seq - ep0 ? ep : seq) + 1u;
-  // copies still in flight (a wait that gave up left a product)
+  // copies still in flight (of a product that the last sum ended or a wait that gave up kept from running)
   for (unsigned k = 0; k < g.offen; ++k) {
     bar_warte(a, sh, &sh.bar[warp][g.stufe], g.par);
     if (++g.stufe == g.stufen) {

@@ -35,7 +35,6 @@ __device__ __forceinline__ uint64_t globaltimer() {
   return t;
 }
 
-constexpr uint64_t kBarrierLimitNs = 4000000000ull;  // 4 s per barrier wait
 // The FP32 operator resolves the relative residual (P^-1 norm) to about
 // 1e-6 on stiff cloth; below that the directions lose conjugacy and a solve
 // can diverge. The mixed form never asks for less.

@@ -37,6 +37,7 @@ constexpr int K3D_STATUS_TIMEOUT = 6;
 // block partials double-buffered (k3d_step.cu).
 constexpr int kRedMax = 4;
 constexpr int kPartialsPerBlock = 2 * kRedMax;
+constexpr uint64_t kBarrierLimitNs = 4000000000ull;  // 4 s per device wait
 
 struct SyncState {
   unsigned count;  // barrier arrivals in this launch (zeroed before each launch)
@@ -220,6 +221,8 @@ struct StepArgs {
   const double* sf_block;
   int64_t sf_cap;
   int ka_blocks, ka_q, ka_smem, ka_rsize;
+  uint64_t frist_ns;   // the longest that a wait of the tiled PCG lasts
+  int64_t stumm_nach;  // for tests: after this iteration a sum waits for a word that no CTA posts (-1: never)
   // bookkeeping
   cudaEvent_t ev_solve0, ev_solve1;  // around the PCG launch (host-side handles)
   SyncState* sync;
