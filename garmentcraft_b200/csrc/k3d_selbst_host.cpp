@@ -39,6 +39,21 @@ void free_all(std::vector<void*>& v) {
   for (void* p : v) cudaFree(p);
   v.clear();
 }
+// A growth of the buffers `v`, whose capacity the caller has set to 0. One that
+// fails leaves none of them, the capacity 0 (at which the next run grows again,
+// whatever it needs) and no last run to read back; the device's error is cleared,
+// so that a run that asks for less is not refused for it.
+template <typename F>
+cudaError_t wachsen(SelbstHost& H, std::vector<void*>& v, F&& f) {
+  free_all(v);
+  const cudaError_t e = f();
+  if (e != cudaSuccess) {
+    free_all(v);
+    H.ran = false;
+    (void)cudaGetLastError();
+  }
+  return e;
+}
 
 }  // namespace
 
@@ -349,96 +364,111 @@ cudaError_t selbst_upload(SelbstHost& H, const k3d_scene* sc, double zusatzdicke
 }
 
 cudaError_t selbst_grow_schnitte(SelbstHost& H, uint32_t cap) {
-  free_all(H.schn);
   SelbstArgs& s = H.s;
-  s.cap_s = cap;
-  cudaError_t e;
-  if ((e = alloc(s.sn_ke, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_t, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_w, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_g, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_wurzel, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_eltern, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_partner, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_sp, size_t(cap) + 1, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_tausch, 6 * size_t(cap), H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_toff, size_t(cap) + 1, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_scan_tmp, selbst_scan_tmp_words(int64_t(cap) + 1), H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.sn_summe, cap, H.schn)) != cudaSuccess) return e;
-  if ((e = alloc(s.klemm, cap, H.schn)) != cudaSuccess) return e;
-  return alloc(s.t_ent, cap, H.schn);
+  s.cap_s = 0;
+  return wachsen(H, H.schn, [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = alloc(s.sn_ke, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_t, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_w, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_g, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_wurzel, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_eltern, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_partner, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_sp, size_t(cap) + 1, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_tausch, 6 * size_t(cap), H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_toff, size_t(cap) + 1, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_scan_tmp, selbst_scan_tmp_words(int64_t(cap) + 1), H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.sn_summe, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.klemm, cap, H.schn)) != cudaSuccess) return e;
+    if ((e = alloc(s.t_ent, cap, H.schn)) != cudaSuccess) return e;
+    s.cap_s = cap;
+    return cudaSuccess;
+  });
 }
 
 cudaError_t selbst_grow_wege(SelbstHost& H, uint32_t cap_p, uint32_t cap_k) {
-  free_all(H.wege);
-  cudaError_t e;
-  H.s.hp2.cap = cap_p;
-  H.s.hk2.cap = cap_k;
-  if ((e = alloc(H.s.hp2.ein, size_t(cap_p), H.wege)) != cudaSuccess) return e;
-  if ((e = alloc(H.s.hp2.elo, size_t(cap_p), H.wege)) != cudaSuccess) return e;
-  if ((e = alloc(H.s.hp2.ehi, size_t(cap_p), H.wege)) != cudaSuccess) return e;
-  if ((e = alloc(H.s.hk2.elo, size_t(cap_k), H.wege)) != cudaSuccess) return e;
-  if ((e = alloc(H.s.hk2.ehi, size_t(cap_k), H.wege)) != cudaSuccess) return e;
-  return alloc(H.s.hk2.ein, size_t(cap_k), H.wege);
+  H.s.hp2.cap = H.s.hk2.cap = 0;
+  return wachsen(H, H.wege, [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = alloc(H.s.hp2.ein, size_t(cap_p), H.wege)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.hp2.elo, size_t(cap_p), H.wege)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.hp2.ehi, size_t(cap_p), H.wege)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.hk2.elo, size_t(cap_k), H.wege)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.hk2.ehi, size_t(cap_k), H.wege)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.hk2.ein, size_t(cap_k), H.wege)) != cudaSuccess) return e;
+    H.s.hp2.cap = cap_p;
+    H.s.hk2.cap = cap_k;
+    return cudaSuccess;
+  });
 }
 
 cudaError_t selbst_grow_edge_hash(SelbstHost& H, uint32_t cap) {
-  free_all(H.hashk);
-  H.s.cap_ek = cap;
-  cudaError_t e;
-  if ((e = alloc(H.s.ebk_lo, size_t(cap), H.hashk)) != cudaSuccess) return e;
-  if ((e = alloc(H.s.ebk_hi, size_t(cap), H.hashk)) != cudaSuccess) return e;
-  return alloc(H.s.ein_k, size_t(cap), H.hashk);
+  H.s.cap_ek = 0;
+  return wachsen(H, H.hashk, [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = alloc(H.s.ebk_lo, size_t(cap), H.hashk)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.ebk_hi, size_t(cap), H.hashk)) != cudaSuccess) return e;
+    if ((e = alloc(H.s.ein_k, size_t(cap), H.hashk)) != cudaSuccess) return e;
+    H.s.cap_ek = cap;
+    return cudaSuccess;
+  });
 }
 
 cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap) {
-  free_all(H.pairs);
   SelbstArgs& s = H.s;
-  s.cap_pairs = cap;
-  s.cap_inc = 5u * cap;
-  cudaError_t e;
-  if ((e = alloc(s.pr_idx, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_src, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_w, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_nab, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_ruhe, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_kf, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_b0, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_b1, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_ga, cap, H.pairs)) != cudaSuccess) return e;
-  char* bR = nullptr;
-  if ((e = alloc(bR, size_t(cap) * 8 * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
-  s.pr_bR = bR;
-  char* wR = nullptr;
-  if ((e = alloc(wR, size_t(cap) * 4 * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
-  s.pr_wR = wR;
-  if ((e = alloc(s.pr_x5, cap, H.pairs)) != cudaSuccess) return e;
-  if ((e = alloc(s.pr_g5, cap, H.pairs)) != cudaSuccess) return e;
-  char* g5R = nullptr;
-  if ((e = alloc(g5R, size_t(cap) * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
-  s.pr_g5R = g5R;
-  if ((e = alloc(s.inc_pos, size_t(8) * cap, H.pairs)) != cudaSuccess) return e;
-  // the per-entry products are in the PCG's vector precision, which is FP64
-  // also where the operator copies are FP32 (K3D_MIXED_STORAGE)
-  char* out = nullptr;
-  if ((e = alloc(out, size_t(s.cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
-  s.inc_out = out;
-  return alloc(s.inc_ent, size_t(s.cap_inc), H.pairs);
+  s.cap_pairs = s.cap_inc = 0;
+  return wachsen(H, H.pairs, [&]() -> cudaError_t {
+    const uint32_t cap_inc = 5u * cap;
+    cudaError_t e;
+    if ((e = alloc(s.pr_idx, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_src, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_w, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_nab, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_ruhe, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_kf, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_b0, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_b1, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_ga, cap, H.pairs)) != cudaSuccess) return e;
+    char* bR = nullptr;
+    if ((e = alloc(bR, size_t(cap) * 8 * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
+    s.pr_bR = bR;
+    char* wR = nullptr;
+    if ((e = alloc(wR, size_t(cap) * 4 * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
+    s.pr_wR = wR;
+    if ((e = alloc(s.pr_x5, cap, H.pairs)) != cudaSuccess) return e;
+    if ((e = alloc(s.pr_g5, cap, H.pairs)) != cudaSuccess) return e;
+    char* g5R = nullptr;
+    if ((e = alloc(g5R, size_t(cap) * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
+    s.pr_g5R = g5R;
+    if ((e = alloc(s.inc_pos, size_t(8) * cap, H.pairs)) != cudaSuccess) return e;
+    // the per-entry products are in the PCG's vector precision, which is FP64
+    // also where the operator copies are FP32 (K3D_MIXED_STORAGE)
+    char* out = nullptr;
+    if ((e = alloc(out, size_t(cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
+    s.inc_out = out;
+    if ((e = alloc(s.inc_ent, size_t(cap_inc), H.pairs)) != cudaSuccess) return e;
+    s.cap_pairs = cap;
+    s.cap_inc = cap_inc;
+    return cudaSuccess;
+  });
 }
 
 cudaError_t selbst_grow_zeilen(SelbstHost& H, uint32_t cap) {
-  free_all(H.sf);
   SelbstArgs& s = H.s;
-  const size_t n = size_t(s.n);
-  cudaError_t e;
-  if ((e = alloc(s.sf_nr, n + 1, H.sf)) != cudaSuccess) return e;
-  if ((e = alloc(s.sf_anf, n, H.sf)) != cudaSuccess) return e;
-  if ((e = alloc(s.sf_anz, n, H.sf)) != cudaSuccess) return e;
-  if ((e = alloc(s.sf_spalte, size_t(cap), H.sf)) != cudaSuccess) return e;
-  if ((e = alloc(s.sf_block, size_t(cap) * 6, H.sf)) != cudaSuccess) return e;
-  s.cap_sf = cap;
   s.zeilen = 1;
-  return cudaSuccess;
+  s.cap_sf = 0;
+  return wachsen(H, H.sf, [&]() -> cudaError_t {
+    const size_t n = size_t(s.n);
+    cudaError_t e;
+    if ((e = alloc(s.sf_nr, n + 1, H.sf)) != cudaSuccess) return e;
+    if ((e = alloc(s.sf_anf, n, H.sf)) != cudaSuccess) return e;
+    if ((e = alloc(s.sf_anz, n, H.sf)) != cudaSuccess) return e;
+    if ((e = alloc(s.sf_spalte, size_t(cap), H.sf)) != cudaSuccess) return e;
+    if ((e = alloc(s.sf_block, size_t(cap) * 6, H.sf)) != cudaSuccess) return e;
+    s.cap_sf = cap;
+    return cudaSuccess;
+  });
 }
 
 cudaError_t selbst_set_naht_ruhe(SelbstHost& H, const double* ruhe, int64_t n_naht, cudaStream_t st) {
@@ -463,7 +493,7 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
   if ((e = cudaMemcpyAsync(z, s.zahl, sizeof(z), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   if (z[SZ_HASH_P] > s.cap_ep) return cudaErrorInvalidValue;  // cannot happen: 8 buckets per point box
-  if (z[SZ_HASH_K] > s.cap_ek) {
+  if (z[SZ_HASH_K] > s.cap_ek || s.cap_ek == 0) {
     const uint64_t want = uint64_t(z[SZ_HASH_K]) + z[SZ_HASH_K] / 2 + 1024;
     if ((e = selbst_grow_edge_hash(H, uint32_t(std::min<uint64_t>(want, 0xffffffffu)))) != cudaSuccess) return e;
   }
@@ -475,14 +505,14 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   if (z[SZ_HASH_S] > s.hs.cap) return cudaErrorInvalidValue;  // cannot happen: 27 buckets per triangle box
   const uint32_t n_s = z[SZ_SCHNITTE];
-  if (n_s > s.cap_s) {
+  if (n_s > s.cap_s || s.cap_s == 0) {
     const uint64_t want = uint64_t(n_s) + n_s / 2 + 1024;
     if (want > 0x0fffffffu) return cudaErrorMemoryAllocation;
     if ((e = selbst_grow_schnitte(H, uint32_t(want))) != cudaSuccess) return e;
   }
   // the proximity pairs, then one push spring per intersection
   const uint64_t paare = uint64_t(z[SZ_PAARE_PT]) + z[SZ_PAARE_KK], federn = paare + n_s;
-  if (federn > s.cap_pairs) {
+  if (federn > s.cap_pairs || s.cap_pairs == 0) {
     const uint64_t want = federn + federn / 2 + 1024;
     if (want > 0x1fffffffu) return cudaErrorMemoryAllocation;
     if ((e = selbst_grow_pairs(H, uint32_t(want))) != cudaSuccess) return e;
@@ -531,7 +561,7 @@ cudaError_t selbst_stoss_run(SelbstHost& H, double* x, const double* nrm_fest, i
   uint32_t z[SZ_COUNT];
   if ((e = cudaMemcpyAsync(z, s.zahl, sizeof(z), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-  if (z[SZ_HASH_P2] > s.hp2.cap || z[SZ_HASH_K2] > s.hk2.cap) {
+  if (z[SZ_HASH_P2] > s.hp2.cap || z[SZ_HASH_K2] > s.hk2.cap || s.hp2.cap == 0) {
     const uint64_t wp = std::max<uint64_t>(s.hp2.cap, uint64_t(z[SZ_HASH_P2]) + z[SZ_HASH_P2] / 2 + 1024);
     const uint64_t wk = std::max<uint64_t>(s.hk2.cap, uint64_t(z[SZ_HASH_K2]) + z[SZ_HASH_K2] / 2 + 1024);
     if (wp > 0x7fffffffu || wk > 0x7fffffffu) return cudaErrorMemoryAllocation;
