@@ -860,8 +860,7 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
     if (n >= (int64_t(1) << 30) || s->n_dreiecke >= (int64_t(1) << 31))
       return fail(h, K3D_BAD_ARGUMENT, "scene too large for the self-collision stage");
     K3D_CUDA(h, selbst_upload(h->sc, s, h->p.selbst_zusatzdicke, h->p.selbst_steifigkeit, int(R), a.x, a.v, cv.masse,
-                              cv.w, cv.reib, st));
-    if (pat.kachel) K3D_CUDA(h, selbst_grow_zeilen(h->sc, uint32_t(4 * n + 1024)));
+                              cv.w, cv.reib, pat.kachel, st));
   }
 
   a.n = n;

@@ -1189,6 +1189,60 @@ __global__ void __launch_bounds__(kT) inc_pos_kernel(const __grid_constant__ Sel
 // 14 a row. A warp a row: its lanes load 32 entries at a time, which then pass
 // in list order, and each lane keeps one neighbour; further neighbours take
 // another sweep. Sums in FP64 in list order, so the same bits on every run.
+//
+// A row's room is four neighbours an entry, which needs no count. Where that is
+// much for the mesh (selbst_run) the neighbours are counted first: up to
+// kNachbarn of them exactly, those beyond once for each coupling.
+constexpr uint32_t kNachbarn = 512;
+template <typename R>
+__global__ void __launch_bounds__(kT) sf_zaehlen_kernel(const __grid_constant__ SelbstArgs s) {
+  __shared__ uint32_t liste[kT / 32][kNachbarn];
+  const int64_t i = (int64_t(blockIdx.x) * kT + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i > s.n) return;
+  uint32_t* da = liste[threadIdx.x >> 5];
+  const uint32_t e0 = i < s.n ? s.inc_off[i] : 0u, e1 = i < s.n ? min(s.inc_off[i + 1], s.cap_inc) : 0u;
+  const R4<R>* wR = static_cast<const R4<R>*>(s.pr_wR);
+  const R* g5R = static_cast<const R*>(s.pr_g5R);
+  uint32_t zahl = 0, mehr = 0;
+  for (uint32_t c = e0; c < e1; c += 32) {
+    uint32_t ix[5] = {0, 0, 0, 0, 0}, gegen = 0;
+    if (c + lane < e1) {
+      const uint32_t ent = s.inc_ent[c + lane], q = ent >> 3, k = ent & 7u;
+      const uint4 id = s.pr_idx[q];
+      const R4<R> w4 = wR[q];
+      const R g[5] = {w4.x, w4.y, w4.z, w4.w, g5R[q]};
+      const uint32_t p[5] = {id.x, id.y, id.z, id.w, s.pr_x5[q]};
+      const R gk = k == 0 ? g[0] : k == 1 ? g[1] : k == 2 ? g[2] : k == 3 ? g[3] : g[4];
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        ix[r] = p[r];
+        if ((gk > R(0) && g[r] < R(0)) || (gk < R(0) && g[r] > R(0))) gegen |= 1u << r;
+      }
+    }
+    const uint32_t mt = min(32u, e1 - c);
+    for (uint32_t t = 0; t < mt; ++t) {
+      const uint32_t gt = __shfl_sync(0xffffffffu, gegen, int(t));
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        const uint32_t j = __shfl_sync(0xffffffffu, ix[r], int(t));
+        if (!((gt >> r) & 1u)) continue;
+        bool bekannt = false;
+        for (uint32_t p = 0; p < zahl && !bekannt; p += 32)
+          bekannt = __any_sync(0xffffffffu, p + lane < zahl && da[p + lane] == j);
+        if (bekannt) continue;
+        if (zahl == kNachbarn) {
+          ++mehr;
+          continue;
+        }
+        if (lane == 0) da[zahl] = j;
+        ++zahl;
+        __syncwarp();
+      }
+    }
+  }
+  if (lane == 0) s.sf_off[i] = e0 < e1 ? 1u + zahl + mehr : 0u;
+}
 __global__ void __launch_bounds__(kT) sf_marke_kernel(const __grid_constant__ SelbstArgs s) {
   SC_FOR(i, s.n + 1) s.sf_nr[i] = i < s.n && s.inc_off[i] != s.inc_off[i + 1] ? 1u : 0u;
 }
@@ -1200,7 +1254,8 @@ __global__ void __launch_bounds__(kT) sf_zeilen_kernel(const __grid_constant__ S
   const uint32_t e0 = s.inc_off[i], e1 = min(s.inc_off[i + 1], s.cap_inc);
   if (e0 >= e1) return;
   const uint32_t zeile = s.sf_nr[i];
-  const size_t anf = 4 * size_t(e0) + zeile;  // at most four neighbours an entry, and the diagonals of the rows before
+  // at most four neighbours an entry, and the diagonals of the rows before
+  const size_t anf = s.sf_genau ? size_t(s.sf_off[i]) : 4 * size_t(e0) + zeile;
   const size_t cap = s.cap_sf;
   const R4<R>* bR = static_cast<const R4<R>*>(s.pr_bR);
   const R4<R>* wR = static_cast<const R4<R>*>(s.pr_wR);
@@ -2586,10 +2641,23 @@ cudaError_t selbst_paare_und_federn(const SelbstArgs& s, uint32_t n_aktiv_p, uin
   inc_fill_kernel<<<grid_for(pmax), kT, 0, st>>>(s);
   inc_sort_kernel<<<grid_for(s.n), kT, 0, st>>>(s);
   if ((e = lang_sort(s.inc_off, s.inc_ent, s.n, st)) != cudaSuccess) return e;
-  if (!s.zeilen) {
-    inc_pos_kernel<<<grid_for(int64_t(s.cap_inc)), kT, 0, st>>>(s);
-    return cudaGetLastError();
-  }
+  if (!s.zeilen) inc_pos_kernel<<<grid_for(int64_t(s.cap_inc)), kT, 0, st>>>(s);
+  return cudaGetLastError();
+}
+
+cudaError_t selbst_zeilen_zaehlen(const SelbstArgs& s, cudaStream_t st) {
+  const unsigned blk = unsigned((s.n + 1 + kT / 32 - 1) / (kT / 32));
+  if (s.rsize == 4)
+    sf_zaehlen_kernel<float><<<blk, kT, 0, st>>>(s);
+  else
+    sf_zaehlen_kernel<double><<<blk, kT, 0, st>>>(s);
+  cudaError_t e;
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return scan(s.sf_off, s.n + 1, s.scan_tmp, &s.zahl[SZ_ZEILEN], st);
+}
+
+cudaError_t selbst_zeilen(const SelbstArgs& s, cudaStream_t st) {
+  cudaError_t e;
   sf_marke_kernel<<<grid_for(s.n + 1), kT, 0, st>>>(s);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = scan(s.sf_nr, s.n + 1, s.scan_tmp, nullptr, st)) != cudaSuccess) return e;

@@ -38,6 +38,7 @@ enum SelbstZahl : int {
   SZ_ARBEIT_S = 20,   // the intersection count pass's next edge
   SZ_ARBEIT_PD = 21,  // the heavy point-triangle impact search's next list entry
   SZ_ARBEIT_KK = 22,  // the heavy edge-edge impact search's next list entry
+  SZ_ZEILEN = 23,     // room of the springs' rows, where it is counted
   SZ_COUNT = 24
 };
 
@@ -106,11 +107,14 @@ struct SelbstArgs {
   uint32_t cap_inc;
   uint32_t* inc_pos;  // per (spring << 3 | slot): its entry index, all ones for a zero weight
   void* inc_out;      // per entry: the PCG's spring product of that slot, R4
-  // the springs as rows of merged blocks, for the tiled PCG (zeilen != 0): row
-  // k of the points with entries has sf_anz[k] blocks from sf_anf[k] on, the
-  // diagonal first; sf_nr: per point its row, then the rows' count (n + 1)
-  int zeilen;
+  // the springs as rows of merged blocks, for the tiled PCG (zeilen != 0; inc_pos
+  // and inc_out are not there then): row k of the points with entries has
+  // sf_anz[k] blocks from sf_anf[k] on, the diagonal first; sf_nr: per point its
+  // row, then the rows' count (n + 1); sf_off: per point the start of its room
+  // where that is counted (sf_genau; n + 1)
+  int zeilen, sf_genau;
   uint32_t cap_sf;
+  uint32_t* sf_off;
   uint32_t *sf_nr, *sf_anf, *sf_anz, *sf_spalte;
   double* sf_block;  // symmetric blocks (xx, yy, zz, xy, xz, yz): 6 planes of cap_sf
   int32_t* slot_of;  // damping scratch per point: its shared-memory slot, -1 between batches
@@ -167,6 +171,10 @@ cudaError_t selbst_hash_fuellen_und_paare_zaehlen(const SelbstArgs& s, cudaStrea
 // n_s: the intersections (counter SZ_SCHNITTE, at most cap_s)
 cudaError_t selbst_paare_und_federn(const SelbstArgs& s, uint32_t n_aktiv_p, uint32_t n_aktiv_s, uint32_t n_s,
                                     cudaStream_t st);
+// The springs' rows, after the part above: the room that they take (into
+// sf_off, and the sum into the counter SZ_ZEILEN), and the rows.
+cudaError_t selbst_zeilen_zaehlen(const SelbstArgs& s, cudaStream_t st);
+cudaError_t selbst_zeilen(const SelbstArgs& s, cudaStream_t st);
 int selbst_launches_per_run(bool zeilen);
 // Impacts after the step's integration, in two parts with a host read of the
 // path hashes' entry counts between them.

@@ -55,6 +55,8 @@ cudaError_t wachsen(SelbstHost& H, std::vector<void*>& v, F&& f) {
   return e;
 }
 
+constexpr uint64_t kZeilenFrei = 128;  // selbst_run
+
 }  // namespace
 
 void selbst_free(SelbstHost& H) {
@@ -70,10 +72,11 @@ void selbst_free(SelbstHost& H) {
 
 cudaError_t selbst_upload(SelbstHost& H, const k3d_scene* sc, double zusatzdicke, double steifigkeit, int rsize,
                           const double* x, double* v, const double* masse, const double* w, const double* reib,
-                          cudaStream_t st) {
+                          bool zeilen, cudaStream_t st) {
   selbst_free(H);
   SelbstArgs& s = H.s;
   std::memset(&s, 0, sizeof(s));
+  s.zeilen = zeilen ? 1 : 0;
   const int64_t n = sc->n_punkte, nd = sc->n_dreiecke;
   s.n = n;
   s.nd = nd;
@@ -359,6 +362,7 @@ cudaError_t selbst_upload(SelbstHost& H, const k3d_scene* sc, double zusatzdicke
   if ((e = selbst_grow_pairs(H, uint32_t(std::min<int64_t>(std::max<int64_t>(n, 1024), 0x3fffffff)))) !=
       cudaSuccess)
     return e;
+  if (zeilen && (e = selbst_grow_zeilen(H, uint32_t(4 * n + 1024))) != cudaSuccess) return e;
   H.on = true;
   return cudaStreamSynchronize(st);
 }
@@ -441,12 +445,16 @@ cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap) {
     char* g5R = nullptr;
     if ((e = alloc(g5R, size_t(cap) * size_t(s.rsize), H.pairs)) != cudaSuccess) return e;
     s.pr_g5R = g5R;
-    if ((e = alloc(s.inc_pos, size_t(8) * cap, H.pairs)) != cudaSuccess) return e;
-    // the per-entry products are in the PCG's vector precision, which is FP64
-    // also where the operator copies are FP32 (K3D_MIXED_STORAGE)
-    char* out = nullptr;
-    if ((e = alloc(out, size_t(cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
-    s.inc_out = out;
+    s.inc_pos = nullptr;
+    s.inc_out = nullptr;
+    if (!s.zeilen) {
+      if ((e = alloc(s.inc_pos, size_t(8) * cap, H.pairs)) != cudaSuccess) return e;
+      // the per-entry products are in the PCG's vector precision, which is FP64
+      // also where the operator copies are FP32 (K3D_MIXED_STORAGE)
+      char* out = nullptr;
+      if ((e = alloc(out, size_t(cap_inc) * 4 * sizeof(double), H.pairs)) != cudaSuccess) return e;
+      s.inc_out = out;
+    }
     if ((e = alloc(s.inc_ent, size_t(cap_inc), H.pairs)) != cudaSuccess) return e;
     s.cap_pairs = cap;
     s.cap_inc = cap_inc;
@@ -456,12 +464,12 @@ cudaError_t selbst_grow_pairs(SelbstHost& H, uint32_t cap) {
 
 cudaError_t selbst_grow_zeilen(SelbstHost& H, uint32_t cap) {
   SelbstArgs& s = H.s;
-  s.zeilen = 1;
   s.cap_sf = 0;
   return wachsen(H, H.sf, [&]() -> cudaError_t {
     const size_t n = size_t(s.n);
     cudaError_t e;
     if ((e = alloc(s.sf_nr, n + 1, H.sf)) != cudaSuccess) return e;
+    if ((e = alloc(s.sf_off, n + 1, H.sf)) != cudaSuccess) return e;
     if ((e = alloc(s.sf_anf, n, H.sf)) != cudaSuccess) return e;
     if ((e = alloc(s.sf_anz, n, H.sf)) != cudaSuccess) return e;
     if ((e = alloc(s.sf_spalte, size_t(cap), H.sf)) != cudaSuccess) return e;
@@ -517,17 +525,27 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
     if (want > 0x1fffffffu) return cudaErrorMemoryAllocation;
     if ((e = selbst_grow_pairs(H, uint32_t(want))) != cudaSuccess) return e;
   }
-  if (s.zeilen) {  // at most four blocks for each nonzero slot, and a diagonal for each point
+  // Room for the rows: at most four blocks for each nonzero slot, and a diagonal
+  // for each point. Up to kZeilenFrei blocks a point that much is kept; where the
+  // springs are denser they share most of their points, and the blocks are
+  // counted below, with another host read. 7.3 k points with 1.7 million pairs,
+  // all of the stage's growing buffers: 2,087 bytes a pair without the count, 623
+  // with it, 838 for the launch over ELL rows; two layers in contact have 56
+  // blocks a point by the bound, the garment 6.
+  s.sf_genau = 0;
+  if (s.zeilen) {
     const uint64_t most = 4 * (4 * paare + 5 * uint64_t(n_s)) + uint64_t(s.n);
-    if (most > s.cap_sf) {
-      const uint64_t want = most + most / 2;
+    s.sf_genau = most > std::max(uint64_t(s.cap_sf), kZeilenFrei * uint64_t(s.n)) ? 1 : 0;
+    if ((most > s.cap_sf && !s.sf_genau) || s.cap_sf == 0) {
+      const uint64_t want = s.sf_genau ? 4 * uint64_t(s.n) + 1024 : most + most / 2;
       if (want > 0xffffffffu) return cudaErrorMemoryAllocation;
       if ((e = selbst_grow_zeilen(H, uint32_t(want))) != cudaSuccess) return e;
     }
   }
   if ((e = cudaMemsetAsync(s.inc_off, 0, sizeof(uint32_t) * (size_t(s.n) + 1), st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(s.inc_cur, 0, sizeof(uint32_t) * size_t(s.n), st)) != cudaSuccess) return e;
-  if (federn > 0 && (e = cudaMemsetAsync(s.inc_pos, 0xff, sizeof(uint32_t) * 8 * size_t(federn), st)) != cudaSuccess)
+  if (s.inc_pos && federn > 0 &&
+      (e = cudaMemsetAsync(s.inc_pos, 0xff, sizeof(uint32_t) * 8 * size_t(federn), st)) != cudaSuccess)
     return e;
   if ((e = cudaMemsetAsync(s.hat, 0, size_t(std::max<int64_t>(s.nd, 1)), st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(s.klemm, 0, size_t(s.cap_s), st)) != cudaSuccess) return e;
@@ -535,13 +553,28 @@ cudaError_t selbst_run(SelbstHost& H, double h, cudaStream_t st, int& launches) 
   if ((e = cudaMemsetAsync(s.t_cur, 0, sizeof(uint32_t) * size_t(std::max<int64_t>(s.nd, 1)), st)) != cudaSuccess)
     return e;
   if ((e = selbst_paare_und_federn(s, z[SZ_AKTIV_P], z[SZ_AKTIV_S], n_s, st)) != cudaSuccess) return e;
+  launches += selbst_launches_per_run(s.zeilen != 0);
+  if (s.zeilen) {
+    for (int versuch = 0; s.sf_genau && versuch < 2; ++versuch) {  // again after a growth, which frees the starts
+      uint32_t bloecke = 0;
+      if ((e = selbst_zeilen_zaehlen(s, st)) != cudaSuccess) return e;
+      launches += 4;
+      if ((e = cudaMemcpyAsync(&bloecke, &s.zahl[SZ_ZEILEN], sizeof(bloecke), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+        return e;
+      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+      if (bloecke <= s.cap_sf) break;
+      const uint64_t want = uint64_t(bloecke) + bloecke / 4;
+      if (versuch || want > 0xffffffffu) return cudaErrorMemoryAllocation;
+      if ((e = selbst_grow_zeilen(H, uint32_t(want))) != cudaSuccess) return e;
+    }
+    if ((e = selbst_zeilen(s, st)) != cudaSuccess) return e;
+  }
   H.n_pt = z[SZ_PAARE_PT];
   H.n_kk = z[SZ_PAARE_KK];
   H.n_s = n_s;
   H.naehe_pt += z[SZ_PAARE_PT];
   H.naehe_kk += z[SZ_PAARE_KK];
   H.ran = true;
-  launches += selbst_launches_per_run(s.zeilen != 0);
   return cudaSuccess;
 }
 

@@ -25,10 +25,11 @@ struct SelbstHost {
   uint64_t naehe_pt = 0, naehe_kk = 0;  // pairs since the last statistics reset
 };
 
-// Builds the mesh tables from the scene and allocates the device buffers.
+// Builds the mesh tables from the scene and allocates the device buffers
+// (zeilen: the springs are to be applied as merged rows).
 cudaError_t selbst_upload(SelbstHost& H, const k3d_scene* sc, double zusatzdicke, double steifigkeit, int rsize,
                           const double* x, double* v, const double* masse, const double* w, const double* reib,
-                          cudaStream_t st);
+                          bool zeilen, cudaStream_t st);
 void selbst_free(SelbstHost& H);
 cudaError_t selbst_grow_edge_hash(SelbstHost& H, uint32_t cap);
 cudaError_t selbst_grow_schnitte(SelbstHost& H, uint32_t cap);

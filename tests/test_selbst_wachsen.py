@@ -40,6 +40,8 @@ size_t selbst_scan_tmp_words(int64_t n) { return size_t(n); }
 cudaError_t selbst_hash_zaehlen(const SelbstArgs&, cudaStream_t) { return cudaSuccess; }
 cudaError_t selbst_hash_fuellen_und_paare_zaehlen(const SelbstArgs&, cudaStream_t) { return cudaSuccess; }
 cudaError_t selbst_paare_und_federn(const SelbstArgs&, uint32_t, uint32_t, uint32_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t selbst_zeilen_zaehlen(const SelbstArgs&, cudaStream_t) { return cudaSuccess; }
+cudaError_t selbst_zeilen(const SelbstArgs&, cudaStream_t) { return cudaSuccess; }
 int selbst_launches_per_run(bool) { return 0; }
 cudaError_t selbst_stoss_zaehlen(const SelbstArgs&, cudaStream_t) { return cudaSuccess; }
 cudaError_t selbst_stoss_antwort(const SelbstArgs&, int, unsigned long long*, cudaStream_t) { return cudaSuccess; }
