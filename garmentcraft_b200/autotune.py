@@ -4,15 +4,17 @@ whose solver has a single CPU form).
 The step has three launch choices that change its speed but not its
 arithmetic beyond the summation order of the grid reductions:
 
-* ``pcg_threads`` -- the CTA size of the persistent PCG launch: 512 threads
-  (one CTA per SM, 128 registers a thread), 256 (two CTAs per SM, the same
-  registers; twice the CTAs at every grid barrier) or 1024 (one CTA per SM,
-  64 registers a thread, so the kernel spills; twice the warps to hide the
-  row products' load latency).
+* ``pcg_threads`` -- the persistent PCG launch and its CTA size. 512 threads
+  (one CTA per SM, 128 registers a thread): the tiled PCG, and the launch over
+  ELL rows where a tile does not fit or the vectors are FP32. 256 (two CTAs per
+  SM, the same registers; twice the CTAs at every grid barrier) or 1024 (one
+  CTA per SM, 64 registers a thread, so the kernel spills; twice the warps to
+  hide the row products' load latency): the launch over ELL rows.
 * ``pcg_bloecke`` -- CTAs of the persistent PCG launch. Every PCG iteration
-  passes two grid barriers whose cost grows with the CTAs that arrive; a
-  small drape has too little work per iteration to hide it, so fewer CTAs
-  win there, while a large drape needs every SM for its row products.
+  has two grid sums whose cost grows with the CTAs; a small drape has too
+  little work per iteration to hide it, so fewer CTAs win there, while a
+  large drape needs every SM for its row products (and the tiled PCG every
+  SM's shared memory: on fewer CTAs its tiles may not fit).
 * ``graph`` -- replaying a frame's launches as one CUDA graph, which removes
   the host launch cost between the short kernels of a substep (not with
   self-collision, whose stage reads counts back between launches).
@@ -21,7 +23,8 @@ arithmetic beyond the summation order of the grid reductions:
 caller's own scene (the same
 frames from the same state, device time from CUDA events), keeps the fastest
 and caches it in a JSON file keyed by the device, the precision and the
-scene's size, so the sweep runs once per shape.
+scene's size, so the sweep runs once per shape. A record holds the launch forms
+it chose among (``FORMEN``); one of another library's forms is timed again.
 """
 from __future__ import annotations
 
@@ -35,6 +38,7 @@ from .szene import Szene
 
 CACHE_ENV = "GARMENTCRAFT_B200_TUNE"
 THREADS = (512, 256, 1024)  # CTA sizes the library is built for
+FORMEN = "kachel 512, ell 512 256 1024"  # what they launch; another text when that changes
 
 
 def cache_pfad() -> str:
@@ -104,8 +108,8 @@ def abstimmen(s: Szene, param: ImplizitParameter | None = None, bilder: int = 3,
     del probe
     key = schluessel(geraet, param, s)
     daten = _lesen(pfad)
-    if not neu and key in daten:
-        rec = daten[key]
+    rec = daten.get(key)
+    if not neu and rec is not None and rec.get("formen") == FORMEN:
         return _gewaehlt(param, rec), rec
     inst = _instanzen(s)
     graphen = (False,) if param.selbstkollision else (False, True)
@@ -133,7 +137,8 @@ def abstimmen(s: Szene, param: ImplizitParameter | None = None, bilder: int = 3,
             del cg
     sieger = min(zeiten, key=lambda z: z["ms_je_bild"])
     rec = {"pcg_threads": sieger["pcg_threads"], "pcg_bloecke": sieger["pcg_bloecke"], "graph": sieger["graph"],
-           "ms_je_bild": sieger["ms_je_bild"], "kandidaten": zeiten, "bilder": bilder}
+           "ms_je_bild": sieger["ms_je_bild"], "kandidaten": zeiten, "bilder": bilder,
+           "formen": FORMEN}
     daten[key] = rec
     _schreiben(pfad, daten)
     return _gewaehlt(param, rec), rec

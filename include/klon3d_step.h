@@ -65,15 +65,20 @@ typedef struct k3d_params {
   int32_t koerperpunkt_durchgaenge;   /* body points against cloth triangles: passes per step (implizit.rs:479), default 0 = off */
   int32_t pcg_bloecke;                /* no reference counterpart: CTAs of the persistent PCG launch, at most one
                                          per SM times the CTAs that fit; 0 (default) = that maximum. Fewer CTAs
-                                         make each grid barrier cheaper, which pays on small drapes */
+                                         make each grid sum cheaper, which pays on small drapes, and the tiled
+                                         PCG's tiles larger (they may not fit then, see pcg_threads) */
   double koerperpunkt_tiefe;          /* m below a body point a triangle is still lifted (implizit.rs:481), default 0.01 */
   int32_t graph;                      /* no reference counterpart: 1 = each frame's launches are captured once as a
                                          CUDA graph and replayed while their arguments stay the same (recaptured
                                          when they change, e.g. a moving body); not with self-collision, whose
                                          stage reads counts back between launches. The per-frame PCG time of
                                          k3d_last_solve_ms stays 0 then. Default 0 */
-  int32_t pcg_threads;                /* no reference counterpart: threads per CTA of the persistent PCG launch,
-                                         256 (two CTAs per SM), 512 or 1024 (one per SM); 0 (default) = 512 */
+  int32_t pcg_threads;                /* no reference counterpart: threads per CTA of the persistent PCG launch;
+                                         0 (default) = 512. With 512 and FP64 vectors (K3D_FP64,
+                                         K3D_MIXED_STORAGE) it is the tiled PCG, one tile of the mesh per CTA,
+                                         where the tiles fit the SMs' shared memory; else, and with 256 (two CTAs
+                                         per SM) or 1024, the launch over rows in global memory. The two differ
+                                         in the order of sums */
 } k3d_params;
 
 /* Simparameter (sim/src/szene.rs:96-126), the part the implicit step reads. */
