@@ -43,6 +43,10 @@ self-collision proximity stage on and off (see garment_leg). ``mesh`` is the
 body mesh as a collider: voxelisation, nearest queries, segment tests and the
 sheet step on an exact mesh body (see mesh_leg).
 
+The JSON line on stdout holds the headline and the main figure of each leg in
+under 2,800 characters (see line_of), as its readers keep the end of the output
+only; the whole record, every candidate and check, goes to stderr as one line.
+
 Multi-GPU: the step of one drape does not shard (a global Krylov solve), so
 ``--gpus N`` runs N independent replicas, one per rank, with no collective on
 the data path; value = total vertex-steps / max over ranks of the time.
@@ -674,6 +678,58 @@ class Clocks:
                 "reasons": reasons, "samples": len(rows)}
 
 
+def rounded(o, digits=5):
+    """`o` with its floats to `digits` significant digits."""
+    if isinstance(o, dict):
+        return {k: rounded(v, digits) for k, v in o.items()}
+    if isinstance(o, (list, tuple)):
+        return [rounded(v, digits) for v in o]
+    return float(f"{o:.{digits}g}") if isinstance(o, float) and math.isfinite(o) else o
+
+
+def line_of(full):
+    """The line on stdout: the headline's keys as they are, and of each leg in
+    `full` its main figures, rounded."""
+    def of(d, *keys):
+        return {k: d[k] for k in keys if d and k in d}
+
+    out = {k: v for k, v in full.items() if k in (
+        "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+        "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks")}
+    out["roofline"] = rounded(of(full.get("roofline"), "bound", "achieved", "peak", "unit", "frac", "kernel"))
+    legs = of(full, "cg_iterations_per_step", "pcg_us_per_iteration")
+    for form in ("fp64", "mixed_fp32_vectors"):
+        if form in full:
+            legs[form + "_ms_per_step"] = full[form]["ms_per_step"]
+    if "mixed_vs_fp64" in full:
+        m = full["mixed_vs_fp64"]
+        err = {f: max(e["max"] for e in es) for f, es in m["one_step_error"]["errors"].items()}
+        legs["mixed_vs_fp64"] = {"speedup": m["speedup"], "one_step_max_err": err,
+                                 "err_100_steps": m["rel_pos_err_after_100_steps"]}
+    if "batched" in full:
+        legs["batched"] = of(full["batched"]["batched_mixed"], "value", "ms_per_step") | of(
+            full["batched"], "batched_vs_per_instance")
+    if "adjoint" in full:
+        a = full["adjoint"]
+        legs["adjoint"] = of(a, "forward_ms", "backward_ms", "backward_forward") | {
+            "gradient_rel_err": a["gradient_check"]["max_best_rel_err"]}
+    if "garment" in full:
+        g = full["garment"]
+        legs["garment"] = {k + "_ms": g[k]["ms_per_step"] for k in (
+            "selfcollision_mixed_storage", "selfcollision_fp64", "no_selfcollision_mixed_storage",
+            "no_selfcollision_fp64")}
+        legs["garment"]["e2e_value"] = g["e2e"]["value"]
+    if "mesh" in full:
+        q = full["mesh"]
+        legs["mesh"] = {"nearest_ms": q["nearest"]["ms_device"], "nearest_e2e_ms": q["nearest"]["e2e"]["ms"],
+                        "sdf_3cm_ms": q["sdf_band_3cm"]["ms_device"], "step_mesh_body_ms": q["step_mesh_body"]["ms_per_step"],
+                        "step_grid_body_ms": q["step_grid_body"]["ms_per_step"]}
+    if "cpu_baseline" in full:
+        legs["cpu_baseline"] = of(full["cpu_baseline"], "value", "unit", "cores", "kind")
+    out.update(rounded(legs))
+    return out
+
+
 def read_peaks():
     try:
         return json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -874,7 +930,8 @@ def main():
             return
         s, cpu = reference_leg(a.n, a.warmup, a.steps)
         line = {"impl": "reference", "metric": METRIC, "value": cpu["value"], "unit": UNIT, "n_gpus": a.gpus,
-                "steps": a.steps, "warmup": a.warmup, "higher_is_better": True, "scaling": "weak",
+                "steps": a.steps, "warmup": a.warmup, "ms_per_step": 1e3 * s.n / cpu["value"],
+                "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f64", "data": "synthetic",
                 "config": workload_config(a.n, s, {"precision": "fp64 (CPU)",
                                                    "l2": "not applicable: one host thread, no device"}),
@@ -1014,7 +1071,8 @@ def main():
     if rank == 0 and world == 1 and not a.no_cpu:
         line["cpu_baseline"] = cpu_sample(a.n, a.warmup, a.steps, a.cpu_seconds, torch)
     if rank == 0:
-        print(json.dumps(line))
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(line_of(line)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
