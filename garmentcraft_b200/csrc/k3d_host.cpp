@@ -48,6 +48,7 @@ struct k3d_solver {
   int blocks = 0;
   uint64_t frist_ns = kBarrierLimitNs;  // StepArgs
   int64_t stumm_nach = -1;
+  int64_t form[4] = {0, 0, 0, 0};  // the PCG launch of the uploaded scene (k3d_test_form)
   size_t ka_smem = 0;  // shared memory a CTA of the tiled PCG takes (0: the launch over ELL rows)
   size_t rsize = 8;  // operator records, assembled blocks, preconditioner
   size_t vsize = 8;  // the PCG's vectors
@@ -655,6 +656,13 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
   pat.kachel = h->ka_smem > 0 && kachelplan(sp, s->x, io, nbk, R, federn, h->ka_smem, kachel_kopf_bytes(), pat.plan) &&
                kachel_bereit(int(R), federn, pat.plan.q, h->ka_smem);
   if (pat.kachel) nbk = pat.plan.nblk;
+  std::fill(h->form, h->form + 4, 0);
+  if (pat.kachel) {
+    h->form[0] = pat.plan.q;
+    h->form[1] = pat.plan.blocks;
+    h->form[2] = int64_t(pat.plan.slabs);
+    for (const uint4& q : pat.plan.slice) h->form[3] += q.y;
+  }
   if (!build_pattern(el, sp, np, pat)) return fail(h, K3D_BAD_ARGUMENT, "scene too large for the block pattern");
 
   // element constants
@@ -1640,8 +1648,12 @@ k3d_status k3d_adjoint_backward(k3d_solver* h, const double* gx, const double* g
   return K3D_OK;
 }
 
-// For the library's tests, not part of the ABI that the headers declare: the
-// tiled PCG's waits last `sekunden` at most, and after iteration `nach` (-1: never)
+// For the library's tests, not part of the ABI that the headers declare. The PCG
+// launch of the uploaded scene: the tiled one's rows a thread (0: the launch over
+// ELL rows), its tiles, slabs and streamed slabs.
+void k3d_test_form(const k3d_solver* h, int64_t out[4]) { std::copy(h->form, h->form + 4, out); }
+
+// The tiled PCG's waits last `sekunden` at most, and after iteration `nach` (-1: never)
 // one of a solve's sums waits for a word that nobody posts.
 void k3d_test_wait(k3d_solver* h, double sekunden, int64_t nach) {
   h->frist_ns = uint64_t(sekunden * 1e9);

@@ -84,7 +84,9 @@ struct Kachelplan {
 // each. False where a tile does not fit: more than kKachelZeilen rows a
 // thread, local columns beyond 16 bits, or no room in `smem` bytes (`kopf` of
 // them the header) for the least ring and the slabs that are left over beside
-// it.
+// it. On a B200's 148 CTAs a regular sheet (13 blocks a row) so fits up to some
+// 227 k points with FP32 blocks, where the two slabs of a grip leave the odd one of
+// every slice over, and beyond 266 k with FP64 blocks.
 //
 // A group of up to kKachelNatur points, and every instance of a batch, keeps
 // the rows and sums of the launch over ELL rows (CTA b, thread t: the rows
