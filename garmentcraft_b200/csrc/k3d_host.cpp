@@ -48,6 +48,8 @@ struct k3d_solver {
   int blocks = 0;
   uint64_t frist_ns = kBarrierLimitNs;  // StepArgs
   int64_t stumm_nach = -1;
+  uint64_t folge = 0;      // no word of the tiled PCG carries a greater sequence number
+  bool erfassung = false;  // the launches are being captured (frame_graph)
   int64_t form[4] = {0, 0, 0, 0};  // the PCG launch of the uploaded scene (k3d_test_form)
   size_t ka_smem = 0;  // shared memory a CTA of the tiled PCG takes (0: the launch over ELL rows)
   size_t rsize = 8;  // operator records, assembled blocks, preconditioner
@@ -657,6 +659,7 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
                kachel_bereit(int(R), federn, pat.plan.q, h->ka_smem);
   if (pat.kachel) nbk = pat.plan.nblk;
   std::fill(h->form, h->form + 4, 0);
+  h->folge = 0;
   if (pat.kachel) {
     h->form[0] = pat.plan.q;
     h->form[1] = pat.plan.blocks;
@@ -888,6 +891,35 @@ k3d_status k3d_upload_scene(k3d_solver* h, const k3d_scene* s) {
 
 }  // extern "C"
 
+// The words and sequence numbers of the tiled PCG as at upload. On the handle's
+// own stream, which the next launch follows (it does not wait for the legacy stream).
+static k3d_status worte_neu(k3d_solver* h) {
+  K3D_CUDA(h, cudaMemsetAsync(h->a.ka_wort, 0, sizeof(ulonglong2) * (h->p.selbstkollision ? 12 : 6) * size_t(h->n),
+                              h->stream));
+  K3D_CUDA(h, cudaMemsetAsync(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte),
+                              h->stream));
+  K3D_CUDA(h, cudaMemsetAsync(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp), h->stream));
+  h->folge = 0;
+  return K3D_OK;
+}
+
+// Room for the sequence numbers of the next `starts` launches: each takes at most
+// two passes of two sums an iteration and a few more. They are 32 bits, some hours
+// of iterations; before they wrap the words start again, as a reader would take a
+// word of 2^32 numbers ago (or one never written, at number 0) for this one's.
+static k3d_status folge_platz(k3d_solver* h, int starts) {
+  if (!h->a.ka_blk) return K3D_OK;
+  constexpr uint64_t kEnde = 0xffffffffu;
+  const uint64_t its = h->p.cg_max > 0 ? std::min<uint64_t>(uint64_t(h->p.cg_max), kEnde / 8) : 0;
+  const uint64_t zahl = uint64_t(starts) * 2 * (2 * its + 8);
+  if (h->folge + zahl > kEnde) {
+    k3d_status st = worte_neu(h);
+    if (st != K3D_OK) return st;
+  }
+  h->folge += zahl;
+  return K3D_OK;
+}
+
 // Fills the per-launch fields and launches one step kernel.
 // The per-launch fields of the handle's StepArgs: step constants and the
 // bodies moved by t_bodies from their frame-start positions.
@@ -949,6 +981,10 @@ static k3d_status launch(k3d_solver* h, int mode, double t_bodies, bool need_loa
     if (es != cudaSuccess) return cuda_fail(h, es, "self-collision stage");
   }
   selbst_step_args(h->sc, a);
+  if (!h->erfassung) {
+    k3d_status st = folge_platz(h, 1);
+    if (st != K3D_OK) return st;
+  }
   cudaError_t e = launch_step(a, h->p.precision, h->blocks, h->stream, launched);
   h->launches += launched;
   if (e != cudaSuccess) return cuda_fail(h, e, "step kernel launch");
@@ -977,15 +1013,10 @@ static k3d_status check_sync(k3d_solver* h) {
   SyncState ss;
   K3D_CUDA(h, cudaMemcpy(&ss, h->a.sync, sizeof(ss), cudaMemcpyDeviceToHost));
   if (ss.error != 0) {
-    // on the handle's own stream, which the next launch follows (it does not
-    // wait for the legacy stream)
     K3D_CUDA(h, cudaMemsetAsync(&h->a.sync->error, 0, sizeof(int), h->stream));
     if (h->a.ka_blk) {  // the sequence numbers of a launch that gave up start again
-      K3D_CUDA(h, cudaMemsetAsync(h->a.ka_wort, 0, sizeof(ulonglong2) * (h->p.selbstkollision ? 12 : 6) * size_t(h->n),
-                                  h->stream));
-      K3D_CUDA(h, cudaMemsetAsync(h->a.ka_summe, 0, sizeof(ulonglong2) * 4 * size_t(kKachelKopien) * size_t(kKachelWorte),
-                                  h->stream));
-      K3D_CUDA(h, cudaMemsetAsync(h->a.grp_cnt, 0, sizeof(unsigned) * 32 * size_t(h->n_grp), h->stream));
+      k3d_status st = worte_neu(h);
+      if (st != K3D_OK) return st;
     }
     return fail(h, K3D_TIMEOUT, "a device barrier wait ran out of time");
   }
@@ -1062,7 +1093,9 @@ static k3d_status frame_graph(k3d_solver* h) {
     K3D_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     const int64_t l0 = h->launches;
     k3d_status st = K3D_OK;
+    h->erfassung = true;
     for (int k = 0; k < sub && st == K3D_OK; ++k) st = launch(h, MODE_STEP, double(k + 1) * hs, false);
+    h->erfassung = false;
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
     if (st != K3D_OK || ec != cudaSuccess) {
@@ -1092,6 +1125,8 @@ static k3d_status frame_graph(k3d_solver* h) {
     }
     h->gkey = std::move(key);
   }
+  k3d_status sf = folge_platz(h, sub);
+  if (sf != K3D_OK) return sf;
   K3D_CUDA(h, cudaGraphLaunch(h->gexec, h->stream));
   h->launches += h->glaunches;
   h->first_step = false;
@@ -1597,6 +1632,7 @@ k3d_status k3d_adjoint_backward(k3d_solver* h, const double* gx, const double* g
       J.dv = r + 2 * N3;
       J.fn = r + 3 * N3;
       J.flags = reinterpret_cast<const uint32_t*>(r + rec_d);
+      if ((st = folge_platz(h, 1)) != K3D_OK) break;
       int launched = 0;
       cudaError_t e = launch_adjoint_step(a, J, h->blocks, h->stream, launched);
       h->launches += launched;
@@ -1652,6 +1688,15 @@ k3d_status k3d_adjoint_backward(k3d_solver* h, const double* gx, const double* g
 // launch of the uploaded scene: the tiled one's rows a thread (0: the launch over
 // ELL rows), its tiles, slabs and streamed slabs.
 void k3d_test_form(const k3d_solver* h, int64_t out[4]) { std::copy(h->form, h->form + 4, out); }
+
+// Sets the tiled PCG's last sequence number, here and on the device.
+k3d_status k3d_test_folge(k3d_solver* h, uint32_t folge) {
+  const std::vector<unsigned> z(32 * size_t(h->n_grp), folge);
+  K3D_CUDA(h, cudaMemcpyAsync(h->a.grp_cnt, z.data(), sizeof(unsigned) * z.size(), cudaMemcpyHostToDevice, h->stream));
+  K3D_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->folge = folge;
+  return K3D_OK;
+}
 
 // The tiled PCG's waits last `sekunden` at most, and after iteration `nach` (-1: never)
 // one of a solve's sums waits for a word that nobody posts.

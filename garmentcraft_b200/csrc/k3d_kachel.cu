@@ -12,8 +12,10 @@
 //    registers for the whole solve;
 //  * the blocks lie in slabs (32 rows of one warp x one rank, with their
 //    columns). As many slabs as fit stay in shared memory for the whole
-//    launch; the others pass through a ring of bulk copies that each warp
-//    keeps full by itself, its first copies on their way before the sum is in;
+//    launch; the others (of regular sheets from 36 k points FP64 and 66 k FP32
+//    blocks on: 45 % there, 86 % at 160 k FP32, all at 90 k FP64) pass through a
+//    ring of bulk copies that each warp keeps full by itself, its first copies on
+//    their way before the sum is in;
 //  * halo values and the CTAs' partial sums travel as words that carry their
 //    own sequence number beside 32 bits of payload: a reader polls the datum
 //    itself, so an exchange costs one store and one load latency, without
@@ -26,11 +28,14 @@
 // iterations 59.8 -> 33.8 ms; 36 k, FP64, 3320 iterations 36.7 -> 24.7 ms;
 // 100 k, FP64, 5840 iterations 232 -> 129 ms; 66 k, FP32 blocks, 3386
 // iterations 36.6 -> 26.2 ms; 6.6 k, FP64, 50 iterations 0.92 -> 0.61 ms. What
-// is left of an iteration: at one row a thread the two sums and the halo
-// (about 1500 cycles a hop, 2600 where 148 CTAs poll one another) and the row
-// product at 30 cycles a slab (23 shared-memory wavefronts, 18 of the
-// conversion unit); beyond, the slabs that do not fit on the SMs, at 9-10 TB/s
-// from L2.
+// is left of an iteration: the two sums and the halo (about 1500 cycles a hop,
+// 2600 where 148 CTAs poll one another), the row product at 30 cycles a slab (23
+// shared-memory wavefronts, 18 of the conversion unit), the streamed slabs, and
+// the warps' unequal shares: a CTA's slices go to its 16 warps whole, so the
+// longest warp has 1.4 times the mean at 160 k points, 1.5 at 104 k FP64 of a
+// garment, 2.1 at 36 k FP64 (8 warps have none), and ncu puts the warps at
+// barriers first. From L2 come 19.5 MB an iteration in 8.1 us at 66 k points, 98 MB
+// in 19.8 us at 160 k (25 MB of it from memory), 19.8 MB in 8.6 us at 36 k FP64.
 // Self-collision springs come as merged rows of blocks (federzeilen): with the
 // launch over ELL rows, which forms each spring's products and sums them by
 // point, 205 k points with 63 k springs, 3051 iterations, took 217 ms, here

@@ -444,8 +444,9 @@ __device__ __forceinline__ void filt3(const V (&n)[3], V& x, V& y, V& z) {
 // updates) from the FP64 operator. With the FP32 operator the block part of
 // A c follows A c = A w + beta A c_prev: the row product gathers w alone (half
 // the bytes of c and w), and ap keeps S A c_prev between iterations. The FP64
-// form applies A to c directly, as the reference does. Returns false on a
-// barrier error.
+// form applies A to c directly, as the reference does (the tiled PCG too, but for
+// the self-collision springs, whose part of A c it carries along the same way).
+// Returns false on a barrier error.
 template <typename R, typename V, bool SC>
 __device__ bool pcg(const StepArgs& a, const Vec<R, V>& vw, Shared& sh, int64_t& iters, bool& unconverged,
                     bool& breakdown, double& rest) {
